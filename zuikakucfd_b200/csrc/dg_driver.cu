@@ -206,10 +206,7 @@ int zk_dg_setup(zk_ctx* c) {
     s->s0 = (P >= 3) ? -3.0 * std::log10((double)P) : -4.0 * std::log10((double)P);
     s->xpitch = c->g.pitch + 32;
     const int NQ = P + 1, NM = NQ * NQ;
-    cudaError_t e = cudaMalloc(&c->d_phic, sizeof(double) * NM * 4);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(c->d_phic, phic, sizeof(double) * NM * 4, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = cudaMalloc(&s->fx, sizeof(double) * NQ * 4 * (size_t)c->g.ny * s->xpitch);
+    cudaError_t e = cudaMalloc(&s->fx, sizeof(double) * NQ * 4 * (size_t)c->g.ny * s->xpitch);
     if (e == cudaSuccess) e = cudaMalloc(&s->fy, sizeof(double) * NQ * 4 * (size_t)(c->g.ny + 1) * c->g.pitch);
     if (e == cudaSuccess && c->opt.precision == ZK_PREC_MIXED) {
         if (zk::dg_upload_tables_f32(P) != ZK_OK) return zk_internal_fail(ZK_ERR_CUDA, "DG FP32 table upload failed");

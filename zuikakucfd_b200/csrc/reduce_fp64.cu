@@ -56,46 +56,72 @@ __device__ __forceinline__ void block_max_commit(double m, unsigned long long* o
 
 // computeMaxSpeed, src_WENO/fluid.cpp:539-553: all cells, no floors; a NaN
 // speed never wins (spd > umax is false), umax starts at 0.
-__global__ void max_speed_weno_kernel(const double* U, Grid g, double gamma, unsigned long long* out) {
+//
+// Bound: HBM (32 B per cell).  A thread takes two neighbouring cells per
+// 16-byte load of each plane (rows are whole 256-byte lines, so pairs never
+// straddle a row) and finds their column from one 32-bit remainder; with a
+// 64-bit division and 8-byte loads per cell the 2048^2 reduction took 58 us
+// (2.3 TB/s), it takes 34 us
+// in this form, the FP64 divisions and square roots alongside.
+__global__ void __launch_bounds__(256) max_speed_weno_kernel(const double* __restrict__ U, Grid g, double gamma,
+                                                             unsigned long long* out) {
     double umax = 0.0;
-    const size_t n = (size_t)g.ny * g.nx;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n;
-         t += (size_t)gridDim.x * blockDim.x) {
-        const size_t i = t / g.nx, j = t - i * g.nx, k = i * g.pitch + j;
-        double rho = U[k];
-        double u = U[g.plane + k] / rho, v = U[2 * g.plane + k] / rho;
-        double p = (gamma - 1.0) * (U[3 * g.plane + k] - 0.5 * rho * (u * u + v * v));
-        double a = sqrt(gamma * p / rho);
-        double spd = sqrt(u * u + v * v) + a;
-        if (spd > umax) umax = spd;
+    const uint32_t half = (uint32_t)g.pitch / 2, n = (uint32_t)g.ny * half;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int j = 2 * (int)(t % half);
+        if (j >= g.nx) continue;
+        const size_t k = 2 * (size_t)t;
+        const double2 r = *reinterpret_cast<const double2*>(U + k);
+        const double2 mx = *reinterpret_cast<const double2*>(U + g.plane + k);
+        const double2 my = *reinterpret_cast<const double2*>(U + 2 * g.plane + k);
+        const double2 E = *reinterpret_cast<const double2*>(U + 3 * g.plane + k);
+        const double s0 = weno_cell_speed(r.x, mx.x, my.x, E.x, gamma);
+        if (s0 > umax) umax = s0;
+        if (j + 1 < g.nx) {
+            const double s1 = weno_cell_speed(r.y, mx.y, my.y, E.y, gamma);
+            if (s1 > umax) umax = s1;
+        }
     }
     block_max_commit(umax, out);
 }
 
-// computeMaxSpeedDG_omp, src_DG/solver.cpp:26-64: bctype-0 cells of the whole
-// grid, state at the 4 corners (xi,eta) = (-1,-1),(+1,-1),(-1,+1),(+1,+1)
-// through phi2 (corner values of the basis in phic[m][4]), floors 1e-12.
-__global__ void max_speed_dg_kernel(const double* dof, const int8_t* kind, Grid g, int nm,
-                                    double gamma, const double* phic, unsigned long long* out) {
-    double umax = 0.0;
-    const size_t n = (size_t)g.ny * g.nx;
-    const double eps = 1e-12;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n;
-         t += (size_t)gridDim.x * blockDim.x) {
-        const size_t i = t / g.nx, j = t - i * g.nx, k = i * g.pitch + j;
-        if (!(kind[k] & KIND_FLUID)) continue;
-        for (int q = 0; q < 4; ++q) {
-            double U[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int m = 0; m < nm; ++m) {
-                const double b = phic[m * 4 + q];
+// Largest corner wave speed of the DG cell at k, or umax
+// (computeMaxSpeedDG_omp, src_DG/solver.cpp:26-64): the state at the corners
+// (xi, eta) = (-1,-1), (+1,-1), (-1,+1), (+1,+1), summed over the modes in
+// increasing order.  P_n(+1) = 1 and P_n(-1) = (-1)^n exactly, so a mode's
+// corner values are +-1 times its coefficient: every coefficient is read once
+// and enters the four sums by additions alone.
+template <int P>
+__device__ __forceinline__ double dg_corner_speed(const double* __restrict__ dof, size_t plane, size_t k,
+                                                  double gamma, double umax) {
+    constexpr int NQ = P + 1, NM = NQ * NQ;
+    double cs[4][4] = {};
 #pragma unroll
-                for (int c = 0; c < 4; ++c) U[c] += dof[(size_t)(c * nm + m) * g.plane + k] * b;
+    for (int m = 0; m < NM; ++m)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double x = dof[(size_t)(c * NM + m) * plane + k];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const bool neg = (((q & 1) ? 0 : m / NQ) + ((q & 2) ? 0 : m % NQ)) & 1;
+                cs[q][c] += neg ? -x : x;
             }
-            double rho = ref_max(U[0], eps), u = U[1] / rho, v = U[2] / rho;
-            double p = ref_max((gamma - 1.0) * (U[3] - 0.5 * rho * (u * u + v * v)), eps);
-            double a = sqrt(gamma * p / rho);
-            umax = ref_max(umax, sqrt(u * u + v * v) + a);
         }
+    return dg_cell_speed(cs, gamma, umax);
+}
+
+// computeMaxSpeedDG_omp over the bctype-0 cells of the whole grid.  Bound: HBM
+// (32 NM B per cell, read once; with the corners in an outer loop each
+// coefficient was read four times and P=3 at 2048^2 took 975 us, now 323 us).
+template <int P>
+__global__ void __launch_bounds__(256) max_speed_dg_kernel(const double* __restrict__ dof,
+                                                           const int8_t* __restrict__ kind, Grid g, double gamma,
+                                                           unsigned long long* out) {
+    double umax = 0.0;
+    const uint32_t pitch = (uint32_t)g.pitch, n = (uint32_t)g.ny * pitch;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        if ((int)(k % pitch) >= g.nx || !(kind[k] & KIND_FLUID)) continue;
+        umax = dg_corner_speed<P>(dof, g.plane, k, gamma, umax);
     }
     block_max_commit(umax, out);
 }
@@ -153,21 +179,13 @@ __global__ void __launch_bounds__(256) max_speed_batch_kernel(const void* __rest
             if (ctl->state >= BATCH_DONE || ctl->lam_ready) continue;
             const Grid g = it.g;
             const size_t n = (size_t)g.ny * g.nx, c1 = min(n, (size_t)(h.local + 1) * kRedChunk);
-            const double eps = 1e-12, gamma = it.gamma;
             for (size_t c = (size_t)h.local * kRedChunk + threadIdx.x; c < c1; c += blockDim.x) {
                 const size_t i = c / g.nx, j = c - i * g.nx, k = i * g.pitch + j;
                 if (!(it.kind[k] & KIND_FLUID)) continue;
-                for (int q = 0; q < 4; ++q) {
-                    double U[4] = {0.0, 0.0, 0.0, 0.0};
-                    for (int m = 0; m < it.nm; ++m) {
-                        const double b = it.phic[m * 4 + q];
-#pragma unroll
-                        for (int v = 0; v < 4; ++v) U[v] += it.U[0][(size_t)(v * it.nm + m) * g.plane + k] * b;
-                    }
-                    double rho = ref_max(U[0], eps), u = U[1] / rho, v = U[2] / rho;
-                    double p = ref_max((gamma - 1.0) * (U[3] - 0.5 * rho * (u * u + v * v)), eps);
-                    double a = sqrt(gamma * p / rho);
-                    umax = ref_max(umax, sqrt(u * u + v * v) + a);
+                switch (it.nm) {
+                    case 4: umax = dg_corner_speed<1>(it.U[0], g.plane, k, it.gamma, umax); break;
+                    case 9: umax = dg_corner_speed<2>(it.U[0], g.plane, k, it.gamma, umax); break;
+                    default: umax = dg_corner_speed<3>(it.U[0], g.plane, k, it.gamma, umax); break;
                 }
             }
         } else {
@@ -180,11 +198,8 @@ __global__ void __launch_bounds__(256) max_speed_batch_kernel(const void* __rest
             const size_t n = (size_t)g.ny * g.nx, c1 = min(n, (size_t)(h.local + 1) * kRedChunk);
             for (size_t c = (size_t)h.local * kRedChunk + threadIdx.x; c < c1; c += blockDim.x) {
                 const size_t i = c / g.nx, j = c - i * g.nx, k = i * g.pitch + j;
-                double rho = U[k];
-                double u = U[g.plane + k] / rho, v = U[2 * g.plane + k] / rho;
-                double p = (gamma - 1.0) * (U[3 * g.plane + k] - 0.5 * rho * (u * u + v * v));
-                double a = sqrt(gamma * p / rho);
-                double spd = sqrt(u * u + v * v) + a;
+                const double spd =
+                    weno_cell_speed(U[k], U[g.plane + k], U[2 * g.plane + k], U[3 * g.plane + k], gamma);
                 if (spd > umax) umax = spd;
             }
         }
@@ -267,16 +282,21 @@ cudaError_t launch_max_speed_weno(const double* U, const Grid& g, double gamma,
                                   unsigned long long* out, int sms, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(out, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;
-    max_speed_weno_kernel<<<grid_for((size_t)g.ny * g.nx, 256, sms), 256, 0, s>>>(U, g, gamma, out);
+    max_speed_weno_kernel<<<grid_for(g.plane / 2, 256, sms), 256, 0, s>>>(U, g, gamma, out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_max_speed_dg(const double* dof, const int8_t* kind, const Grid& g, int nm,
-                                double gamma, const double* phic, unsigned long long* out, int sms,
-                                cudaStream_t s) {
+cudaError_t launch_max_speed_dg(const double* dof, const int8_t* kind, const Grid& g, int nm, double gamma,
+                                unsigned long long* out, int sms, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(out, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;
-    max_speed_dg_kernel<<<grid_for((size_t)g.ny * g.nx, 256, sms), 256, 0, s>>>(dof, kind, g, nm, gamma, phic, out);
+    const int grid = grid_for(g.plane, 256, sms);
+    switch (nm) {
+        case 4: max_speed_dg_kernel<1><<<grid, 256, 0, s>>>(dof, kind, g, gamma, out); break;
+        case 9: max_speed_dg_kernel<2><<<grid, 256, 0, s>>>(dof, kind, g, gamma, out); break;
+        case 16: max_speed_dg_kernel<3><<<grid, 256, 0, s>>>(dof, kind, g, gamma, out); break;
+        default: return cudaErrorInvalidValue;
+    }
     return cudaGetLastError();
 }
 

@@ -43,7 +43,7 @@ void free_device(zk_ctx* c) {
     if (c->step_graph) cudaGraphExecDestroy(c->step_graph);  // it captured the buffers freed below
     c->step_graph = nullptr;
     for (void* p : {(void*)c->Un, (void*)c->S1, (void*)c->S2, (void*)c->kind, (void*)c->gsrc,
-                    (void*)c->d_max, (void*)c->d_status, (void*)c->d_phic, (void*)c->d_tmp,
+                    (void*)c->d_max, (void*)c->d_status, (void*)c->d_tmp,
                     (void*)c->F1, (void*)c->F2})
         if (p) cudaFree(p);
     c->Un = c->S1 = c->S2 = c->d_tmp = nullptr;
@@ -52,7 +52,6 @@ void free_device(zk_ctx* c) {
     c->gsrc = nullptr;
     c->d_max = nullptr;
     c->d_status = nullptr;
-    c->d_phic = nullptr;
 }
 
 }  // namespace
@@ -477,7 +476,7 @@ int zk_max_speed(zk_ctx* c, double* out) {
     if (!out) return fail(ZK_ERR_ARG, "null argument");
     ZK_CUDA(cudaSetDevice(c->opt.device));
     if (c->opt.method == ZK_METHOD_DG) {
-        ZK_CUDA(launch_max_speed_dg(c->Un, c->kind, c->g, c->nm, c->gamma, c->d_phic, c->d_max, c->sms, c->stream));
+        ZK_CUDA(launch_max_speed_dg(c->Un, c->kind, c->g, c->nm, c->gamma, c->d_max, c->sms, c->stream));
     } else {
         ZK_CUDA(launch_max_speed_weno(c->Un, c->g, c->gamma, c->d_max, c->sms, c->stream));
     }

@@ -30,7 +30,6 @@ struct zk_ctx {
     int32_t* gsrc = nullptr;  // fill source (pitched linear index) of ghost cells
     unsigned long long* d_max = nullptr;
     uint32_t* d_status = nullptr;
-    double* d_phic = nullptr;  // DG basis at the 4 cell corners, [NM][4]
 
     CUtensorMap tmap[3];  // TMA maps over Un, S1, S2 (mixed WENO path)
 

@@ -42,9 +42,8 @@ cudaError_t launch_fill_ghosts(double* U, const int8_t* kind, const int32_t* gsr
                                int nvar, int nm, int sms, cudaStream_t s);
 cudaError_t launch_max_speed_weno(const double* U, const Grid& g, double gamma,
                                   unsigned long long* out, int sms, cudaStream_t s);
-cudaError_t launch_max_speed_dg(const double* dof, const int8_t* kind, const Grid& g, int nm,
-                                double gamma, const double* phic, unsigned long long* out, int sms,
-                                cudaStream_t s);
+cudaError_t launch_max_speed_dg(const double* dof, const int8_t* kind, const Grid& g, int nm, double gamma,
+                                unsigned long long* out, int sms, cudaStream_t s);
 cudaError_t launch_recover(const double* U, const Grid& g, int nm, double gamma, double* prim,
                            int sms, cudaStream_t s);
 cudaError_t launch_mach(const double* U, const Grid& g, int nm, double gamma, double* mach, double* speed, int sms,
