@@ -385,7 +385,7 @@ def measure_single(name: str, args, rank: int, world: int, local: int, pg, e2e: 
             kname = "weno_stage_fp64_kernel" if f64 else "weno_stage_mixed_kernel"
         else:
             # the mixed stage kernel the context's tuner chose (threads per cell)
-            kname = ("dg_face_kernel x2 + dg_cell_kernel (one stage)" if f64
+            kname = ("dg_face_kernel + dg_cell_kernel (one stage)" if f64
                      else DG_MIXED_KERNEL.get(pth["tpc"], "dg_stage_mixed_kernel"))
         if prec == "fp64_fma":
             kname = ("weno_stage_fp64_kernel, FMA-contracted build" if w["method"] == "weno"

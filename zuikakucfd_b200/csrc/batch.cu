@@ -803,7 +803,7 @@ int zk_batch_group_tile(zk_batch* b, int g, int* tile_rows, int* tile_cols, int*
         threads = rows * cols * dg_variant_tpc(G.variant);
     } else {
         cols = kDgCellBlock;  // the FP64 DG cell pass
-        threads = cols;
+        threads = cols * (G.order + 1);
     }
     if (tile_rows) *tile_rows = rows;
     if (tile_cols) *tile_cols = cols;

@@ -59,8 +59,8 @@ constexpr int kDgVariants = 4;
 constexpr int dg_variant_rows(int v) { return kDgTileRows[v & 1]; }
 constexpr int dg_variant_tpc(int v) { return 1 + (v >> 1); }
 constexpr int kDgDefaultVariant = 1;  // 32 x 4, one thread per cell
-// Row segment of the FP64 DG cell pass (one thread per cell).
-constexpr int kDgCellBlock = 64;
+// Row segment of the FP64 DG passes (order + 1 threads per cell in the cell pass).
+constexpr int kDgCellBlock = 32;
 
 // CTAs per SM to promise in __launch_bounds__ for a persistent stage kernel:
 // as many as keep every thread within the register share of `thread_budget`
@@ -136,21 +136,23 @@ __device__ __forceinline__ double weno_cell_speed(double r, double mx, double my
     return __dadd_rn(__dsqrt_rn(q), a);
 }
 
-// Largest corner wave speed of one DG cell (computeMaxSpeedDG_omp,
-// src_DG/solver.cpp:26-64): U at the corners accumulated over the modes in
-// increasing order, floors 1e-12.  cs[k][c] = variable c at corner k.
-__device__ __forceinline__ double dg_cell_speed(const double (&cs)[4][4], double gamma, double umax) {
+// Wave speed of a DG corner state U, or umax (computeMaxSpeedDG_omp,
+// src_DG/solver.cpp:26-64; floors 1e-12).
+__device__ __forceinline__ double dg_state_speed(const double (&U)[4], double gamma, double umax) {
     const double eps = 1e-12;
+    const double rho = ref_max(U[0], eps);
+    const double u = __ddiv_rn(U[1], rho), v = __ddiv_rn(U[2], rho);
+    const double q = __dadd_rn(__dmul_rn(u, u), __dmul_rn(v, v));
+    const double p = ref_max(__dmul_rn(__dsub_rn(gamma, 1.0), __dsub_rn(U[3], __dmul_rn(__dmul_rn(0.5, rho), q))), eps);
+    const double a = __dsqrt_rn(__ddiv_rn(__dmul_rn(gamma, p), rho));
+    return ref_max(umax, __dadd_rn(__dsqrt_rn(q), a));
+}
+
+// Largest corner wave speed of one DG cell: U at the corners accumulated over
+// the modes in increasing order.  cs[k][c] = variable c at corner k.
+__device__ __forceinline__ double dg_cell_speed(const double (&cs)[4][4], double gamma, double umax) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const double rho = ref_max(cs[k][0], eps);
-        const double u = __ddiv_rn(cs[k][1], rho), v = __ddiv_rn(cs[k][2], rho);
-        const double q = __dadd_rn(__dmul_rn(u, u), __dmul_rn(v, v));
-        const double p =
-            ref_max(__dmul_rn(__dsub_rn(gamma, 1.0), __dsub_rn(cs[k][3], __dmul_rn(__dmul_rn(0.5, rho), q))), eps);
-        const double a = __dsqrt_rn(__ddiv_rn(__dmul_rn(gamma, p), rho));
-        umax = ref_max(umax, __dadd_rn(__dsqrt_rn(q), a));
-    }
+    for (int k = 0; k < 4; ++k) umax = dg_state_speed(cs[k], gamma, umax);
     return umax;
 }
 

@@ -1,18 +1,18 @@
 // Discontinuous Galerkin P=1..3 stage, FP64, the reference's arithmetic op
 // for op (compiled with --fmad=false, like weno_fp64.cu).
 //
-// Per RK stage two kernels:
-//   dg_face_kernel<P, DIR>  every x (DIR=0) / y (DIR=1) interface flux ONCE:
-//                           traces of both cells at the NQ Gauss points of the
-//                           face (ghost neighbours gathered through the fill
-//                           source map), HLLC or HLL; the reference computes
-//                           each face twice from identical inputs.
-//   dg_cell_kernel<P>       per cell: volume quadrature, the four face
-//                           integrals in the reference's order (right, left,
-//                           bottom, top), inverse-mass scaling, the Shu-Osher
-//                           combine and the Persson + Zhang-Shu limiter, all in
-//                           registers; ghosts get the combine of their filled
-//                           value, exactly as the whole-array reference does.
+// Per RK stage two kernels, both on segments of 32 columns of a row:
+//   dg_face_kernel<P>   every x and y interface flux ONCE: traces of both cells
+//                       at the NQ Gauss points of the face (ghost neighbours
+//                       gathered through the fill source map), HLLC or HLL; the
+//                       reference computes each face twice from identical
+//                       inputs.
+//   dg_cell_kernel<P>   P + 1 threads per cell: volume quadrature, the four
+//                       face integrals in the reference's order (right, left,
+//                       bottom, top), inverse-mass scaling, the Shu-Osher
+//                       combine and the Persson + Zhang-Shu limiter; ghosts get
+//                       the combine of their filled value, exactly as the
+//                       whole-array reference does.
 // Basis values are tabulated on the host (no FMA contraction) with the
 // reference's own expressions and kept in __constant__ memory, one table set
 // per P.
@@ -251,97 +251,169 @@ __device__ __forceinline__ CellRef cell_ref(const DGArgs& a, size_t k) {
     return {(size_t)a.gsrc[k], kd == KIND_SLIP_X ? 1 : (kd == KIND_SLIP_Y ? 2 : -1)};
 }
 
-// Traces of one cell at the NQ points of one side: U[q][c] = sum_m dof*phi.
-template <int P>
-__device__ __forceinline__ void cell_traces(const DGArgs& a, CellRef r, const double (&tr)[DG_MAXNQ][DG_MAXNM],
-                                            double (&U)[P + 1][4]) {
-    constexpr int NQ = P + 1, NM = NQ * NQ;
-#pragma unroll
-    for (int q = 0; q < NQ; ++q)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) U[q][c] = 0.0;
-#pragma unroll
-    for (int m = 0; m < NM; ++m) {
-        double d[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const double x = a.cur[(size_t)(c * NM + m) * a.g.plane + r.k];
-            d[c] = (r.neg == c) ? -x : x;
-        }
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) U[q][c] += d[c] * tr[q][m];
-    }
+__device__ __forceinline__ void copy8_async(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// One thread per interface.  DIR 0: x face (i, jf) between cells (i, jf-1)
-// and (i, jf); DIR 1: y face (if, j) between (if-1, j) above and (if, j) below.
-// Faces (i, jb + threadIdx.x).
-template <int P, int DIR>
-__device__ __forceinline__ void face_row(const DGArgs& a, int jb, int i) {
-    constexpr int NQ = P + 1;
+// ---- interface fluxes --------------------------------------------------------------
+// One CTA takes the 32 x faces on the left of cells (i, j0 .. j0+31) and the
+// 32 y faces above them; a warp takes one direction and QP of the NQ Gauss
+// points of its 32 faces.  Both rows of cells are staged in shared memory once
+// and serve both directions (a thread per face and direction read each cell
+// twice from L2, and its 4 NQ traces took 128-146 registers: 4 CTAs of 4 warps
+// per SM, FP64 pipe 40-45%).
+template <int P>
+struct FaceTile {
+    static constexpr int NQ = P + 1, NM = NQ * NQ;
+    static constexpr int QP = P == 3 ? 2 : NQ;  // Gauss points per thread
+    static constexpr int NWD = NQ / QP;         // warps per direction
+    static constexpr int NTHREAD = 64 * NWD;
+    double lo[4 * NM][34];  // row i, columns j0-1 .. j0+31
+    double up[4 * NM][32];  // row i-1, columns j0 .. j0+31
+};
+
+template <int P>
+__device__ __forceinline__ void face_tile(const DGArgs& a, int j0, int i, FaceTile<P>& S) {
+    using F = FaceTile<P>;
+    constexpr int NM = F::NM, QP = F::QP, NW = F::NTHREAD / 32;
     const DGTab& T = c_dgtab[P - 1];
     const int ny = a.g.ny, nx = a.g.nx, pitch = a.g.pitch;
-    const int j = jb + threadIdx.x;
-    size_t kl, kr;  // the two cells
-    if (DIR == 0) {
-        if (j < 1 || j >= nx || i >= ny) return;
-        kl = (size_t)i * pitch + (j - 1);
-        kr = (size_t)i * pitch + j;
-    } else {
-        if (j >= nx || i < 1 || i >= ny) return;
-        kl = (size_t)(i - 1) * pitch + j;
-        kr = (size_t)i * pitch + j;
+    const size_t plane = a.g.plane;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int j = j0 + lane;                      // < pitch: the padding columns are passive cells
+    const size_t k = (size_t)i * pitch + j;
+    const size_t kl = j > 0 ? k - 1 : k;          // j = 0 has no x face
+    const bool cu = (a.kind[k] & KIND_MASK) == KIND_UPDATED;
+    const bool need_x = j > 0 && j < nx && (cu || (a.kind[kl] & KIND_MASK) == KIND_UPDATED);
+    const bool need_y = j < nx && (cu || (a.kind[k - pitch] & KIND_MASK) == KIND_UPDATED);
+    if (!__any_sync(0xffffffffu, need_x || need_y)) return;  // the same cells in every warp
+    const CellRef rc = cell_ref(a, k), ru = cell_ref(a, k - pitch);
+    for (int v = w; v < 4 * NM; v += NW) {
+        copy8_async(&S.lo[v][lane + 1], a.cur + (size_t)v * plane + rc.k);
+        copy8_async(&S.up[v][lane], a.cur + (size_t)v * plane + ru.k);
     }
-    if ((a.kind[kl] & KIND_MASK) != KIND_UPDATED && (a.kind[kr] & KIND_MASK) != KIND_UPDATED) return;
-    double UL[NQ][4], UR[NQ][4];
-    cell_traces<P>(a, cell_ref(a, kl), T.tr[DIR == 0 ? 0 : 2], UL);
-    cell_traces<P>(a, cell_ref(a, kr), T.tr[DIR == 0 ? 1 : 3], UR);
-    const size_t qstride = (DIR == 0) ? (size_t)ny * a.xpitch : (size_t)(ny + 1) * pitch;
-    const size_t o = (DIR == 0) ? (size_t)i * a.xpitch + j : (size_t)i * pitch + j;
-    double* F = (DIR == 0) ? a.fx : a.fy;
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        double f[4];
-        if (DIR == 0) {
-            if (a.hll) hlle_dg(UL[q], UR[q], a.gamma, f);
-            else hllc_dg(UL[q], UR[q], a.gamma, f);
-        } else {
-            // normal (y) momentum into slot 1, and back (src_DG/fluid.cpp:772-774)
-            double l[4] = {UL[q][0], UL[q][2], UL[q][1], UL[q][3]};
-            double r[4] = {UR[q][0], UR[q][2], UR[q][1], UR[q][3]};
-            double g[4];
-            if (a.hll) hlle_dg(l, r, a.gamma, g);
-            else hllc_dg(l, r, a.gamma, g);
-            f[0] = g[0]; f[1] = g[2]; f[2] = g[1]; f[3] = g[3];
+    const CellRef rl = cell_ref(a, j0 > 0 ? k - lane - 1 : k - lane);  // the column left of the tile
+    for (int v = threadIdx.x; v < 4 * NM; v += F::NTHREAD) copy8_async(&S.lo[v][0], a.cur + (size_t)v * plane + rl.k);
+    copy_commit();
+    copy_wait<0>();
+    // slip walls: each thread negates what it copied
+    if (rc.neg >= 0 || ru.neg >= 0)
+        for (int v = w; v < 4 * NM; v += NW) {
+            if (rc.neg == v / NM) S.lo[v][lane + 1] = -S.lo[v][lane + 1];
+            if (ru.neg == v / NM) S.up[v][lane] = -S.up[v][lane];
         }
+    if (rl.neg >= 0)
+        for (int v = threadIdx.x; v < 4 * NM; v += F::NTHREAD)
+            if (rl.neg == v / NM) S.lo[v][0] = -S.lo[v][0];
+    __syncthreads();
+
+    const bool ydir = w >= F::NWD;
+    const int q0 = (ydir ? w - F::NWD : w) * QP;
+    if (!(ydir ? need_y : need_x)) return;
+    const double* pl = ydir ? &S.up[0][lane] : &S.lo[0][lane];
+    const int sl = ydir ? 32 : 34;
+    const double* pr = &S.lo[0][lane + 1];
+    const double(*tl)[DG_MAXNM] = T.tr[ydir ? 2 : 0];
+    const double(*tr)[DG_MAXNM] = T.tr[ydir ? 3 : 1];
+    double UL[QP][4], UR[QP][4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) F[(size_t)(q * 4 + c) * qstride + o] = f[c];
+    for (int u = 0; u < QP; ++u)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) UL[u][c] = UR[u][c] = 0.0;
+#pragma unroll
+    for (int m = 0; m < NM; ++m)
+#pragma unroll
+        for (int u = 0; u < QP; ++u) {
+            const double bl = tl[q0 + u][m], br = tr[q0 + u][m];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                UL[u][c] += pl[(c * NM + m) * sl] * bl;
+                UR[u][c] += pr[(c * NM + m) * 34] * br;
+            }
+        }
+    const size_t qstride = ydir ? (size_t)(ny + 1) * pitch : (size_t)ny * a.xpitch;
+    double* out = ydir ? a.fy + k : a.fx + (size_t)i * a.xpitch + j;
+#pragma unroll
+    for (int u = 0; u < QP; ++u) {
+        // y faces: normal momentum into slot 1, and back (src_DG/fluid.cpp:772-774)
+        const double l[4] = {UL[u][0], ydir ? UL[u][2] : UL[u][1], ydir ? UL[u][1] : UL[u][2], UL[u][3]};
+        const double r[4] = {UR[u][0], ydir ? UR[u][2] : UR[u][1], ydir ? UR[u][1] : UR[u][2], UR[u][3]};
+        double f[4];
+        if (a.hll) hlle_dg(l, r, a.gamma, f);
+        else hllc_dg(l, r, a.gamma, f);
+        double* o = out + (size_t)((q0 + u) * 4) * qstride;
+        o[0] = f[0];
+        o[qstride] = ydir ? f[2] : f[1];
+        o[2 * qstride] = ydir ? f[1] : f[2];
+        o[3 * qstride] = f[3];
     }
 }
 
-template <int P, int DIR>
-__global__ void __launch_bounds__(128) dg_face_kernel(DGArgs a) {
-    face_row<P, DIR>(a, blockIdx.x * blockDim.x, blockIdx.y);
+template <int P>
+__global__ void __launch_bounds__(FaceTile<P>::NTHREAD) dg_face_kernel(DGArgs a) {
+    __shared__ FaceTile<P> S;
+    face_tile<P>(a, blockIdx.x * 32, 3 + blockIdx.y, S);  // rows 3 .. ny-3 hold every face of an updated cell
 }
 
-// applyLimiter for one cell held in registers (src_DG/fluid.cpp:824-992):
-// Persson modal filter (bctype-0 cells only) then Zhang-Shu positivity.
+// ---- cells ---------------------------------------------------------------------------
+// One CTA takes 32 cells of a row with one thread per cell and px: thread
+// (lane, w) holds the 4 NQ modes m = w NQ .. w NQ + NQ - 1 of cell lane.
+// Each mode's sum over the quadrature points, faces and limiter points keeps
+// the reference's order, so the split changes no bit; what a thread needs from
+// the others (the Euler fluxes at a point, each evaluated once, by warp
+// w = its eta index) goes through shared memory.  A warp's global accesses are
+// whole 256-byte row segments, its table reads are warp-uniform.  With one
+// thread per cell the 64 accumulators of P = 3 spilled 656 bytes and the face
+// fluxes arrived in 16 dependent rounds of loads (P=3 1024^2: 2,093 us, FP64
+// pipe 28%); now 720 us (FP64 pipe 66%).  The same layout at P=2 203x331: 69 ->
+// 32 us.
 template <int P>
-__device__ __forceinline__ void limit_cell(double (&o)[4][(P + 1) * (P + 1)], bool persson, const DGTab& T,
-                                           double gamma, double s0) {
-    constexpr int NM = (P + 1) * (P + 1);
+struct CellTile {
+    static constexpr int NQ = P + 1, NM = NQ * NQ, NTHREAD = 32 * NQ;
+    static constexpr int CH = P == 3 ? 2 : NQ;  // quadrature rows per round of point fluxes
+    double sd[4 * NM][32];      // filled stage input; later the limiter's view of the result
+    double fg[CH * NQ][8][32];  // F and G at the round's points; later the limiter's exchange
+    double fx[4 * NQ][33], fyu[4 * NQ][32], fyd[4 * NQ][32];  // interface fluxes
+};
+
+// applyLimiter (src_DG/fluid.cpp:824-992) on the tile: Persson modal filter
+// (cells with persson set) then Zhang-Shu positivity, on the cells with `in`
+// set.  o = the thread's modes.  Variable c's filter is evaluated by warp
+// c mod NQ, point pt of the 16 positivity points by warp pt mod NQ; minima
+// over the points are exact in any order.  A positivity pass whose outcome is
+// known is skipped: |factor| <= 1, so point values lie within mean +- sum
+// |modes|, and when that lower bound (less a 1e-12 relative margin, 500 times
+// the rounding of a 16-term sum) clears the floor the pass returns exactly 1.
+// Every thread of the CTA calls it; ends with every thread past its reads of S.
+template <int P>
+__device__ __forceinline__ void limit_tile(CellTile<P>& S, double (&o)[4][P + 1], bool in, bool persson,
+                                           const DGTab& T, double gamma, double s0) {
+    constexpr int NQ = P + 1, NM = NQ * NQ, NZ = NQ < 3 ? NQ : 3;
     const double kappa = 1.0, RHO_MIN = 1e-5, P_MIN = 1e-5, EPS = 1e-5;
-    if (persson) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double(*ex)[32] = S.fg[0];  // exchange rows of 32 lanes, through the flux buffer
+    constexpr int FAC = 0, SPR = 4, THR = SPR + 4 * NQ, THP = THR + NQ;
+    static_assert((THP + NQ) * 32 * sizeof(double) <= sizeof(S.fg), "the exchange rows fit the flux buffer");
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) S.sd[c * NM + w * NQ + n][lane] = o[c][n];
+    __syncthreads();
+    for (int c = w; c < 4; c += NQ) {
+        double f = 1.0;
+        if (in && persson) {
             double Etot = 0.0, Ep = 0.0;
 #pragma unroll
             for (int m = 0; m < NM; ++m) {
-                const double x = o[c][m];
+                const double x = S.sd[c * NM + m][lane];
                 Etot += x * x;
-                if (m / (P + 1) == P || m % (P + 1) == P) Ep += x * x;
+                if (m / NQ == P || m % NQ == P) Ep += x * x;
             }
             const double s = log10(Ep / (Etot + EPS));
             if (s > s0) {
@@ -351,170 +423,306 @@ __device__ __forceinline__ void limit_cell(double (&o)[4][(P + 1) * (P + 1)], bo
                     const double r = (s - s0) / kappa;
                     eps = 0.5 * (1.0 + sin(M_PI * (r - 0.5)));
                 }
-#pragma unroll
-                for (int m = 0; m < NM; ++m)
-                    if (m / (P + 1) == P || m % (P + 1) == P) o[c][m] *= (1.0 - eps);
+                f = 1.0 - eps;
             }
         }
+        ex[FAC + c][lane] = f;
     }
-    o[0][0] = ref_max(o[0][0], RHO_MIN);
-    const double rho0 = o[0][0], mx0 = o[1][0], my0 = o[2][0];
-    double E0 = o[3][0];
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const double f = ex[FAC + c][lane];
+        double spread = 0.0;
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) {
+            if (w == P || n == P) {
+                o[c][n] *= f;
+                S.sd[c * NM + w * NQ + n][lane] = o[c][n];
+            }
+            if (w < NZ && n < NZ && (w || n)) spread += fabs(o[c][n]);
+        }
+        ex[SPR + c * NQ + w][lane] = spread;
+    }
+    __syncthreads();
+    // means: density floor, pressure floor through the energy (every warp)
+    const double rho0 = ref_max(S.sd[0][lane], RHO_MIN), mx0 = S.sd[NM][lane], my0 = S.sd[2 * NM][lane];
+    double E0 = S.sd[3 * NM][lane];
     const double p0 = (gamma - 1.0) * (E0 - 0.5 * (mx0 * mx0 + my0 * my0) / rho0);
-    if (p0 < P_MIN) {
-        E0 = P_MIN / (gamma - 1.0) + 0.5 * (mx0 * mx0 + my0 * my0) / rho0;
+    if (p0 < P_MIN) E0 = P_MIN / (gamma - 1.0) + 0.5 * (mx0 * mx0 + my0 * my0) / rho0;
+    if (in && w == 0) {
+        o[0][0] = rho0;
         o[3][0] = E0;
     }
-    double theta_rho = 1.0;
-#pragma unroll 1
-    for (int pt = 0; pt < 16; ++pt) {
-        double rho = 0.0;
+    double sp[4];
 #pragma unroll
-        for (int m = 0; m < NM; ++m) rho += o[0][m] * T.zs[pt][m];
-        if (rho < RHO_MIN) {
-            const double t = (rho0 - RHO_MIN) / (rho0 - rho + EPS);
-            theta_rho = ref_min(theta_rho, t);
-        }
+    for (int c = 0; c < 4; ++c) {
+        sp[c] = ex[SPR + c * NQ][lane];
+#pragma unroll
+        for (int n = 1; n < NQ; ++n) sp[c] += ex[SPR + c * NQ + n][lane];
     }
-    if (theta_rho < 1.0) {
+    double theta_rho = 1.0;
+    const bool rho_pass = in && !(rho0 - sp[0] - 1e-12 * (fabs(rho0) + sp[0]) > RHO_MIN);
+    if (__syncthreads_or(rho_pass)) {
+        double th = 1.0;
+        if (rho_pass)
+#pragma unroll 1
+            for (int pt = w; pt < 16; pt += NQ) {
+                asm volatile("" ::: "memory");  // the modes stay in shared memory
+                double rho = 0.0 + rho0 * T.zs[pt][0];
 #pragma unroll
-        for (int m = 1; m < NM; ++m)
+                for (int m = 1; m < NM; ++m) rho += S.sd[m][lane] * T.zs[pt][m];
+                if (rho < RHO_MIN) th = ref_min(th, (rho0 - RHO_MIN) / (rho0 - rho + EPS));
+            }
+        ex[THR + w][lane] = th;
+        __syncthreads();
 #pragma unroll
-            for (int c = 0; c < 4; ++c) o[c][m] *= theta_rho;
+        for (int n = 0; n < NQ; ++n) theta_rho = ref_min(theta_rho, ex[THR + n][lane]);
+        if (theta_rho < 1.0)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int n = 0; n < NQ; ++n)
+                    if (w || n) {
+                        o[c][n] *= theta_rho;
+                        S.sd[c * NM + w * NQ + n][lane] = o[c][n];
+                    }
+    }
+    const double p_avg = (gamma - 1.0) * (E0 - 0.5 * (mx0 * mx0 + my0 * my0) / rho0);
+    bool p_pass = in;
+    {
+        const double rlo = rho0 - sp[0] - 1e-12 * (fabs(rho0) + sp[0]);
+        if (rlo > RHO_MIN) {  // theta_rho is 1 here
+            const double mx = fabs(mx0) + sp[1], my = fabs(my0) + sp[2];
+            const double ke = 0.5 * (mx * mx + my * my) / rlo;
+            const double plo =
+                (gamma - 1.0) * (E0 - sp[3] - ke) - 1e-12 * (gamma - 1.0) * (fabs(E0) + sp[3] + ke);
+            if (plo > P_MIN) p_pass = false;
+        }
     }
     double theta_p = 1.0;
+    if (__syncthreads_or(p_pass)) {
+        double th = 1.0;
+        if (p_pass)
 #pragma unroll 1
-    for (int pt = 0; pt < 16; ++pt) {
-        double rho = 0.0, mx = 0.0, my = 0.0, E = 0.0;
+            for (int pt = w; pt < 16; pt += NQ) {
+                asm volatile("" ::: "memory");
+                const double f0 = T.zs[pt][0];
+                double rho = 0.0 + rho0 * f0, mx = 0.0 + mx0 * f0, my = 0.0 + my0 * f0, E = 0.0 + E0 * f0;
 #pragma unroll
-        for (int m = 0; m < NM; ++m) {
-            const double phi = T.zs[pt][m];
-            rho += o[0][m] * phi;
-            mx += o[1][m] * phi;
-            my += o[2][m] * phi;
-            E += o[3][m] * phi;
-        }
-        if (rho <= RHO_MIN) continue;
-        const double u = mx / rho, v = my / rho;
-        const double p = (gamma - 1.0) * (E - 0.5 * rho * (u * u + v * v));
-        if (p < P_MIN) {
-            const double p_avg = (gamma - 1.0) * (o[3][0] - 0.5 * (o[1][0] * o[1][0] + o[2][0] * o[2][0]) / o[0][0]);
-            const double t = (p_avg - P_MIN) / (p_avg - p + EPS);
-            theta_p = ref_min(theta_p, t);
-        }
+                for (int m = 1; m < NM; ++m) {
+                    const double phi = T.zs[pt][m];
+                    rho += S.sd[m][lane] * phi;
+                    mx += S.sd[NM + m][lane] * phi;
+                    my += S.sd[2 * NM + m][lane] * phi;
+                    E += S.sd[3 * NM + m][lane] * phi;
+                }
+                if (rho <= RHO_MIN) continue;
+                const double u = mx / rho, v = my / rho;
+                const double p = (gamma - 1.0) * (E - 0.5 * rho * (u * u + v * v));
+                if (p < P_MIN) th = ref_min(th, (p_avg - P_MIN) / (p_avg - p + EPS));
+            }
+        ex[THP + w][lane] = th;
+        __syncthreads();
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) theta_p = ref_min(theta_p, ex[THP + n][lane]);
     }
-    if (theta_p < 1.0) {
+    if (theta_p < 1.0)
 #pragma unroll
-        for (int m = 1; m < NM; ++m)
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) o[c][m] *= theta_p;
-    }
+            for (int n = 0; n < NQ; ++n)
+                if (w || n) o[c][n] *= theta_p;
 }
 
-constexpr int kCellBlock = kDgCellBlock;
-
-// Cells (i, jb + threadIdx.x); sd[v][threadIdx.x] is this thread's (filled)
-// stage input, column-private.  Returns the cell's max corner wave speed when
-// want_lam and the cell is fluid (computeMaxSpeedDG_omp), else 0.
+// Cells (i, j0 .. j0+31).  Returns the thread's max corner wave speed of the
+// fluid cells written when want_lam (computeMaxSpeedDG_omp), else 0.  Ends with
+// every thread past its reads of S, except for a caller's barrier.
 template <int P>
-__device__ __forceinline__ double cell_row(const DGArgs& a, int jb, int i,
-                                           double (&sd)[4 * (P + 1) * (P + 1)][kCellBlock]) {
-    constexpr int NQ = P + 1, NM = NQ * NQ, NV = NQ * NQ;
+__device__ __forceinline__ double cell_tile(const DGArgs& a, int j0, int i, CellTile<P>& S) {
+    using C = CellTile<P>;
+    constexpr int NQ = C::NQ, NM = C::NM, CH = C::CH;
     const DGTab& T = c_dgtab[P - 1];
-    const int t = threadIdx.x;
-    const int j = jb + t;
-    if (j >= a.g.nx) return 0.0;  // no block-wide synchronisation follows
     const int ny = a.g.ny, nx = a.g.nx;
-    const size_t plane = a.g.plane, k = (size_t)i * a.g.pitch + j;
+    const size_t plane = a.g.plane;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int j = j0 + lane;  // < pitch: the padding columns are passive cells
+    const size_t k = (size_t)i * a.g.pitch + j;
     const int8_t kd = a.kind[k] & KIND_MASK;
+    const bool upd = kd == KIND_UPDATED;
+    const bool work = __any_sync(0xffffffffu, upd);  // the same in every warp
     const CellRef r = cell_ref(a, k);
-#pragma unroll
-    for (int v = 0; v < 4 * NM; ++v) {
-        const double x = a.cur[(size_t)v * plane + r.k];
-        sd[v][t] = (r.neg == v / NM) ? -x : x;
+
+    for (int v = w; v < 4 * NM; v += NQ) copy8_async(&S.sd[v][lane], a.cur + (size_t)v * plane + r.k);
+    copy_commit();
+    if (work) {
+        const size_t xq = (size_t)ny * a.xpitch, yq = (size_t)(ny + 1) * a.g.pitch;
+        const double* fx = a.fx + (size_t)i * a.xpitch + j;
+        for (int e = w; e < 4 * NQ; e += NQ) {
+            copy8_async(&S.fx[e][lane], fx + e * xq);
+            if (lane == 31) copy8_async(&S.fx[e][32], fx + e * xq + 1);
+            copy8_async(&S.fyu[e][lane], a.fy + e * yq + k);
+            copy8_async(&S.fyd[e][lane], a.fy + e * yq + k + a.g.pitch);
+        }
     }
-    double o[4][NM];
+    copy_commit();
+    if (a.stage > 0) {  // U^n towards L2; read by the combine
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int n = 0; n < NQ; ++n)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(a.un + (size_t)(c * NM + w * NQ + n) * plane + k));
+    }
+    copy_wait<1>();
+    if (r.neg >= 0)  // slip walls: each thread negates what it copied
+        for (int v = w; v < 4 * NM; v += NQ)
+            if (v / NM == r.neg) S.sd[v][lane] = -S.sd[v][lane];
+    __syncthreads();
+
+    double o[4][NQ];
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int m = 0; m < NM; ++m) o[c][m] = 0.0;
-
-    if (kd == KIND_UPDATED) {
-        // volume integral (src_DG/fluid.cpp:698-718)
+        for (int n = 0; n < NQ; ++n) o[c][n] = 0.0;
+    if (work) {
+        // volume integral (src_DG/fluid.cpp:698-718), CH rows of points at a time
 #pragma unroll 1
-        for (int p = 0; p < NV; ++p) {
-            double U[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int qa0 = 0; qa0 < NQ; qa0 += CH) {
+            double U[CH][4];
 #pragma unroll
-            for (int m = 0; m < NM; ++m) {
-                const double b = T.vphi[p][m];
+            for (int u = 0; u < CH; ++u)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) U[c] += sd[c * NM + m][t] * b;
+                for (int c = 0; c < 4; ++c) U[u][c] = S.sd[c * NM][lane];  // phi_0 = 1
+#pragma unroll
+            for (int m = 1; m < NM; ++m)
+#pragma unroll
+                for (int u = 0; u < CH; ++u) {
+                    const double b = T.vphi[(qa0 + u) * NQ + w][m];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) U[u][c] += S.sd[c * NM + m][lane] * b;
+                }
+#pragma unroll
+            for (int u = 0; u < CH; ++u) {
+                double F[4], G[4];
+                euler_flux(U[u], a.gamma, F, G);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    S.fg[u * NQ + w][c][lane] = F[c];
+                    S.fg[u * NQ + w][4 + c][lane] = G[c];
+                }
             }
-            double F[4], G[4];
-            euler_flux(U, a.gamma, F, G);
-            const double coeff = T.vw[p];
-#pragma unroll
-            for (int m = 0; m < NM; ++m) {
-                const double dxi = T.vdxi[p][m], det = T.vdet[p][m];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) o[c][m] += coeff * (F[c] * dxi + G[c] * det);
-            }
-        }
-        // face integrals: right (-), left (+), bottom (-), top (+) (src_DG/fluid.cpp:731-796)
-        const size_t xq = (size_t)ny * a.xpitch, yq = (size_t)(ny + 1) * a.g.pitch;
-        const size_t xr = (size_t)i * a.xpitch + j + 1, xl = (size_t)i * a.xpitch + j;
-        const size_t yd = (size_t)(i + 1) * a.g.pitch + j, yu = (size_t)i * a.g.pitch + j;
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-            const double* Fb = (f < 2) ? a.fx : a.fy;
-            const size_t qs = (f < 2) ? xq : yq;
-            const size_t o_ = (f == 0) ? xr : (f == 1) ? xl : (f == 2) ? yd : yu;
-            const bool minus = (f == 0 || f == 2);
+            __syncthreads();
+            // terms whose basis derivative is 0 identically (d/dxi at px = 0,
+            // d/deta at py = 0) add +-0 and are left out, but for mode 0, whose
+            // sum still turns NaN on a non-finite flux as the reference's does
 #pragma unroll 1
-            for (int q = 0; q < NQ; ++q) {
-                double Fs[4];
+            for (int pt = 0; pt < CH * NQ; ++pt) {
+                const int p = qa0 * NQ + pt;
+                const double coeff = T.vw[p];
+                double F[4], G[4];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) Fs[c] = Fb[(size_t)(q * 4 + c) * qs + o_];
+                for (int c = 0; c < 4; ++c) {
+                    F[c] = S.fg[pt][c][lane];
+                    G[c] = S.fg[pt][4 + c][lane];
+                }
+                if (w == 0) {
 #pragma unroll
-                for (int m = 0; m < NM; ++m) {
-                    const double bv = T.bv[f][q][m];
+                    for (int c = 0; c < 4; ++c) o[c][0] += coeff * (F[c] * 0.0 + G[c] * 0.0);
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        if (minus) o[c][m] -= bv * Fs[c];
-                        else o[c][m] += bv * Fs[c];
+                    for (int n = 1; n < NQ; ++n) {
+                        const double det = T.vdet[p][n];
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) o[c][n] += coeff * (G[c] * det);
+                    }
+                } else {
+                    const double dx0 = T.vdxi[p][w * NQ];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) o[c][0] += coeff * (F[c] * dx0);
+#pragma unroll
+                    for (int n = 1; n < NQ; ++n) {
+                        const double dxi = T.vdxi[p][w * NQ + n], det = T.vdet[p][w * NQ + n];
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) o[c][n] += coeff * (F[c] * dxi + G[c] * det);
                     }
                 }
+            }
+            if (qa0 + CH < NQ) __syncthreads();
+        }
+        copy_wait<0>();
+        __syncthreads();
+        // face integrals: right (-), left (+), bottom (-), top (+)
+        // (src_DG/fluid.cpp:731-796).  P_n(+1) = 1 and P_n(-1) = (-1)^n exactly,
+        // so an x face's weights are those of px = 0 up to sign, and a y face's
+        // weight is one per thread: its product serves all NQ modes.
+        const bool odd = w & 1;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const double f = S.fx[q * 4 + c][lane + 1];
+#pragma unroll
+                for (int n = 0; n < NQ; ++n) o[c][n] -= T.bv[0][q][n] * f;
+            }
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const double x = S.fx[q * 4 + c][lane], f = odd ? -x : x;
+#pragma unroll
+                for (int n = 0; n < NQ; ++n) o[c][n] += T.bv[0][q][n] * f;
+            }
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const double b = T.bv[2][q][w * NQ];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const double t = b * S.fyd[q * 4 + c][lane];
+#pragma unroll
+                for (int n = 0; n < NQ; ++n) o[c][n] -= t;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const double b = T.bv[2][q][w * NQ];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const double t = b * S.fyu[q * 4 + c][lane];
+#pragma unroll
+                for (int n = 0; n < NQ; ++n) o[c][n] += (n & 1) ? -t : t;
             }
         }
         // inverse mass: (2px+1)(2py+1) * 0.5 / h (src_DG/fluid.cpp:800-804)
 #pragma unroll
-        for (int m = 0; m < NM; ++m) {
-            const double scale = (double)((2 * (m / NQ) + 1) * (2 * (m % NQ) + 1)) * a.inv2h;
+        for (int n = 0; n < NQ; ++n) {
+            const double scale = (double)((2 * w + 1) * (2 * n + 1)) * a.inv2h;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) o[c][m] = o[c][m] * scale;
+            for (int c = 0; c < 4; ++c) o[c][n] = upd ? o[c][n] * scale : 0.0;
         }
     }
 
     if (a.stage == 0) {
+        if (j < nx)
 #pragma unroll
-        for (int v = 0; v < 4 * NM; ++v) a.out[(size_t)v * plane + k] = o[v / NM][v % NM];
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int n = 0; n < NQ; ++n) a.out[(size_t)(c * NM + w * NQ + n) * plane + k] = o[c][n];
         return 0.0;
     }
     // Shu-Osher combine with dt applied (src_DG/fluid.cpp:1024-1026, 1036-1038, 1046-1048)
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int m = 0; m < NM; ++m) {
-            const size_t v = (size_t)(c * NM + m);
-            const double dn = a.un[v * plane + k];
-            const double dd = a.dt * o[c][m];
-            if (a.stage == 1) o[c][m] = dn + dd;
-            else if (a.stage == 2) o[c][m] = 0.75 * dn + 0.25 * (sd[v][t] + dd);
-            else o[c][m] = (1.0 / 3.0) * dn + (2.0 / 3.0) * (sd[v][t] + dd);
+        for (int n = 0; n < NQ; ++n) {
+            const int v = c * NM + w * NQ + n;
+            const double dn = a.un[(size_t)v * plane + k];
+            const double dd = a.dt * o[c][n];
+            const double x = S.sd[v][lane];
+            if (a.stage == 1) o[c][n] = dn + dd;
+            else if (a.stage == 2) o[c][n] = 0.75 * dn + 0.25 * (x + dd);
+            else o[c][n] = (1.0 / 3.0) * dn + (2.0 / 3.0) * (x + dd);
         }
-    if (a.limiter == ZK_LIMITER_REFERENCE && i >= 3 && i < ny - 3 && j >= 3 && j < nx - 3)
-        limit_cell<P>(o, kd == KIND_UPDATED, T, a.gamma, a.s0);
-    if (kd == KIND_UPDATED) {
+    if (a.limiter == ZK_LIMITER_REFERENCE && i >= 3 && i < ny - 3)
+        limit_tile<P>(S, o, j >= 3 && j < nx - 3, upd, T, a.gamma, a.s0);
+    if (upd && w == 0) {
         uint32_t flags = 0;
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -522,27 +730,45 @@ __device__ __forceinline__ double cell_row(const DGArgs& a, int jb, int i,
         if (!(o[0][0] > 0.0)) flags |= STATUS_RHO;
         if (flags) atomicOr(a.status, flags);
     }
+    if (j < nx)
 #pragma unroll
-    for (int v = 0; v < 4 * NM; ++v) a.out[(size_t)v * plane + k] = o[v / NM][v % NM];
-    if (!a.want_lam || !(a.kind[k] & KIND_FLUID)) return 0.0;
-    double cs[4][4] = {};
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int m = 0; m < NM; ++m)
+            for (int n = 0; n < NQ; ++n) a.out[(size_t)(c * NM + w * NQ + n) * plane + k] = o[c][n];
+    if (!a.want_lam) return 0.0;
+    // corner q by warp q mod NQ; corner values of the basis are +-1 (reduce_fp64.cu)
+    __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const double b = a.phic[m * 4 + q];
+    for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) cs[q][c] += o[c][m] * b;
+        for (int n = 0; n < NQ; ++n) S.sd[c * NM + w * NQ + n][lane] = o[c][n];
+    __syncthreads();
+    double umax = 0.0;
+    if (j < nx && (a.kind[k] & KIND_FLUID))
+        for (int q = w; q < 4; q += NQ) {
+            double cs[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int m = 0; m < NM; ++m) {
+                const bool neg = (((q & 1) ? 0 : m / NQ) + ((q & 2) ? 0 : m % NQ)) & 1;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const double x = S.sd[c * NM + m][lane];
+                    cs[c] += neg ? -x : x;
+                }
+            }
+            umax = dg_state_speed(cs, a.gamma, umax);
         }
-    return dg_cell_speed(cs, a.gamma, 0.0);
+    return umax;
 }
 
+// CTAs per SM of the cell kernels: 128, 104 and 80 registers, no spills (P=2:
+// 6 over 5 CTAs +1.2%; P=3: 5 CTAs at 100 registers the same time).
+constexpr int cell_ctas(int P) { return P == 3 ? 4 : P == 2 ? 6 : 12; }
+
 template <int P>
-// at least 6 CTAs per SM (at most 168 registers): +4% on the P=3 stage over
-// the 255-register build with 4 CTAs
-__global__ void __launch_bounds__(kCellBlock, 6) dg_cell_kernel(DGArgs a) {
-    __shared__ double sd[4 * (P + 1) * (P + 1)][kCellBlock];
-    cell_row<P>(a, blockIdx.x * kCellBlock, blockIdx.y, sd);
+__global__ void __launch_bounds__(CellTile<P>::NTHREAD, cell_ctas(P)) dg_cell_kernel(DGArgs a) {
+    __shared__ CellTile<P> S;
+    cell_tile<P>(a, blockIdx.x * 32, blockIdx.y, S);
 }
 
 // Stage-s arguments of batch item `it` (stage s reads U[s-1], writes U[s % 3]).
@@ -571,13 +797,14 @@ __device__ __forceinline__ DGArgs batch_args(const DgItem& it, int stage) {
     return a;
 }
 
-// Persistent face pass of a batch group: a problem's tiles are its x-face
-// rows (ny x ceil(nx/128) segments) followed by its y-face rows.
+// Persistent face pass of a batch group: a problem's tiles are its rows
+// 3 .. ny-3 in segments of 32 columns.
 template <int P>
-__global__ void __launch_bounds__(128) dg_faces_fp64_batch_kernel(const DgItem* __restrict__ items,
-                                                                   const int* __restrict__ dir, int cap, int stage) {
+__global__ void __launch_bounds__(FaceTile<P>::NTHREAD, P == 3 ? 5 : 8) dg_faces_fp64_batch_kernel(
+    const DgItem* __restrict__ items, const int* __restrict__ dir, int cap, int stage) {
+    __shared__ FaceTile<P> S;
     __shared__ DGArgs sa;
-    __shared__ int s_job[4];  // stepping, direction, row, segment start
+    __shared__ int s_job[3];  // stepping, row, segment start
     const int total = __ldg(dir + 1);
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
         if (threadIdx.x == 0) {
@@ -585,29 +812,23 @@ __global__ void __launch_bounds__(128) dg_faces_fp64_batch_kernel(const DgItem* 
             const DgItem& it = items[h.item];
             s_job[0] = it.ctl->stepping;
             if (s_job[0]) {
-                const int segs = (it.g.nx + 127) / 128, per = it.g.ny * segs;
-                const int d = h.local >= per, r = h.local - d * per;
-                s_job[1] = d;
-                s_job[2] = r / segs;
-                s_job[3] = (r - (r / segs) * segs) * 128;
+                const int segs = (it.g.nx + 31) / 32, r = h.local / segs;
+                s_job[1] = 3 + r;
+                s_job[2] = (h.local - r * segs) * 32;
                 sa = batch_args(it, stage);
             }
         }
         __syncthreads();
-        if (s_job[0]) {
-            if (s_job[1] == 0) face_row<P, 0>(sa, s_job[3], s_job[2]);
-            else face_row<P, 1>(sa, s_job[3], s_job[2]);
-        }
+        if (s_job[0]) face_tile<P>(sa, s_job[2], s_job[1], S);
         __syncthreads();
     }
 }
 
-// Persistent cell pass of a batch group: tiles are row segments of kCellBlock cells.
+// Persistent cell pass of a batch group: tiles are row segments of 32 cells.
 template <int P>
-__global__ void __launch_bounds__(kCellBlock, 6) dg_cell_fp64_batch_kernel(const DgItem* __restrict__ items,
-                                                                         const int* __restrict__ dir, int cap,
-                                                                         int stage) {
-    __shared__ double sd[4 * (P + 1) * (P + 1)][kCellBlock];
+__global__ void __launch_bounds__(CellTile<P>::NTHREAD, cell_ctas(P)) dg_cell_fp64_batch_kernel(
+    const DgItem* __restrict__ items, const int* __restrict__ dir, int cap, int stage) {
+    __shared__ CellTile<P> S;
     __shared__ DGArgs sa;
     __shared__ int s_job[3];  // stepping, row, segment start
     __shared__ unsigned long long* s_lam;
@@ -618,16 +839,16 @@ __global__ void __launch_bounds__(kCellBlock, 6) dg_cell_fp64_batch_kernel(const
             const DgItem& it = items[h.item];
             s_job[0] = it.ctl->stepping;
             if (s_job[0]) {
-                const int segs = (it.g.nx + kCellBlock - 1) / kCellBlock;
+                const int segs = (it.g.nx + 31) / 32;
                 s_job[1] = h.local / segs;
-                s_job[2] = (h.local - s_job[1] * segs) * kCellBlock;
+                s_job[2] = (h.local - s_job[1] * segs) * 32;
                 sa = batch_args(it, stage);
                 s_lam = &it.ctl->lam;
             }
         }
         __syncthreads();
         if (s_job[0]) {
-            const double m = cell_row<P>(sa, s_job[2], s_job[1], sd);
+            const double m = cell_tile<P>(sa, s_job[2], s_job[1], S);
             if (stage == 3) block_max_commit_to(m, s_lam);  // the next step's wave speed
         }
         __syncthreads();
@@ -636,32 +857,37 @@ __global__ void __launch_bounds__(kCellBlock, 6) dg_cell_fp64_batch_kernel(const
 
 // applyLimiter alone, in place on the state (src_DG/fluid.cpp:824-992).
 template <int P>
-__global__ void __launch_bounds__(kCellBlock) dg_limit_kernel(DGArgs a) {
-    constexpr int NM = (P + 1) * (P + 1);
-    const int j = blockIdx.x * kCellBlock + threadIdx.x, i = blockIdx.y;
-    const int ny = a.g.ny, nx = a.g.nx;
-    if (!(i >= 3 && i < ny - 3 && j >= 3 && j < nx - 3)) return;
+__global__ void __launch_bounds__(CellTile<P>::NTHREAD) dg_limit_kernel(DGArgs a) {
+    constexpr int NQ = P + 1, NM = NQ * NQ;
+    __shared__ CellTile<P> S;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + lane, i = 3 + blockIdx.y;
+    const bool in = j >= 3 && j < a.g.nx - 3;
     const size_t plane = a.g.plane, k = (size_t)i * a.g.pitch + j;
-    double o[4][NM];
+    double o[4][NQ];
 #pragma unroll
-    for (int v = 0; v < 4 * NM; ++v) o[v / NM][v % NM] = a.out[(size_t)v * plane + k];
-    limit_cell<P>(o, (a.kind[k] & KIND_MASK) == KIND_UPDATED, c_dgtab[P - 1], a.gamma, a.s0);
+    for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int v = 0; v < 4 * NM; ++v) a.out[(size_t)v * plane + k] = o[v / NM][v % NM];
+        for (int n = 0; n < NQ; ++n) o[c][n] = a.out[(size_t)(c * NM + w * NQ + n) * plane + k];
+    limit_tile<P>(S, o, in, (a.kind[k] & KIND_MASK) == KIND_UPDATED, c_dgtab[P - 1], a.gamma, a.s0);
+    if (in)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int n = 0; n < NQ; ++n) a.out[(size_t)(c * NM + w * NQ + n) * plane + k] = o[c][n];
 }
 
 template <int P>
 cudaError_t launch_stage(const DGArgs& a, cudaStream_t s) {
-    const dim3 fb(128);
-    dg_face_kernel<P, 0><<<dim3((a.g.nx + 127) / 128, a.g.ny), fb, 0, s>>>(a);
-    dg_face_kernel<P, 1><<<dim3((a.g.nx + 127) / 128, a.g.ny), fb, 0, s>>>(a);
-    dg_cell_kernel<P><<<dim3((a.g.nx + kCellBlock - 1) / kCellBlock, a.g.ny), kCellBlock, 0, s>>>(a);
+    const int segs = (a.g.nx + 31) / 32;
+    dg_face_kernel<P><<<dim3(segs, a.g.ny - 5), FaceTile<P>::NTHREAD, 0, s>>>(a);
+    dg_cell_kernel<P><<<dim3(segs, a.g.ny), CellTile<P>::NTHREAD, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 template <int P>
 cudaError_t launch_limit(const DGArgs& a, cudaStream_t s) {
-    dg_limit_kernel<P><<<dim3((a.g.nx + kCellBlock - 1) / kCellBlock, a.g.ny), kCellBlock, 0, s>>>(a);
+    dg_limit_kernel<P><<<dim3((a.g.nx + 31) / 32, a.g.ny - 6), CellTile<P>::NTHREAD, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -676,16 +902,14 @@ cudaError_t launch_dg_stage_fp64(int P, const DGArgs& a, cudaStream_t s) {
     }
 }
 
-// Batch tiles per problem: face pass 2 ny ceil(nx/128), cell pass ny ceil(nx/64).
-int dg_fp64_batch_tiles(int pass, int ny, int nx) {
-    return pass == 0 ? 2 * ny * ((nx + 127) / 128) : ny * ((nx + kCellBlock - 1) / kCellBlock);
-}
+// Batch tiles per problem: face pass (ny - 5) ceil(nx/32), cell pass ny ceil(nx/32).
+int dg_fp64_batch_tiles(int pass, int ny, int nx) { return (pass == 0 ? ny - 5 : ny) * ((nx + 31) / 32); }
 
 template <int P>
 cudaError_t launch_batch_p(const DgItem* items, const int* dir_face, const int* dir_cell, int cap, int stage,
                            int grid_face, int grid_cell, cudaStream_t s) {
-    dg_faces_fp64_batch_kernel<P><<<grid_face, 128, 0, s>>>(items, dir_face, cap, stage);
-    dg_cell_fp64_batch_kernel<P><<<grid_cell, kCellBlock, 0, s>>>(items, dir_cell, cap, stage);
+    dg_faces_fp64_batch_kernel<P><<<grid_face, FaceTile<P>::NTHREAD, 0, s>>>(items, dir_face, cap, stage);
+    dg_cell_fp64_batch_kernel<P><<<grid_cell, CellTile<P>::NTHREAD, 0, s>>>(items, dir_cell, cap, stage);
     return cudaGetLastError();
 }
 
@@ -704,12 +928,12 @@ cudaError_t launch_dg_stage_fp64_batch(int P, const DgItem* items, const int* di
 int dg_fp64_batch_occupancy(int P, int pass) {
     int n = 0;
     switch (P * 2 + pass) {
-        case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_faces_fp64_batch_kernel<1>, 128, 0); break;
-        case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_cell_fp64_batch_kernel<1>, kCellBlock, 0); break;
-        case 4: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_faces_fp64_batch_kernel<2>, 128, 0); break;
-        case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_cell_fp64_batch_kernel<2>, kCellBlock, 0); break;
-        case 6: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_faces_fp64_batch_kernel<3>, 128, 0); break;
-        case 7: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_cell_fp64_batch_kernel<3>, kCellBlock, 0); break;
+        case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_faces_fp64_batch_kernel<1>, FaceTile<1>::NTHREAD, 0); break;
+        case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_cell_fp64_batch_kernel<1>, CellTile<1>::NTHREAD, 0); break;
+        case 4: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_faces_fp64_batch_kernel<2>, FaceTile<2>::NTHREAD, 0); break;
+        case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_cell_fp64_batch_kernel<2>, CellTile<2>::NTHREAD, 0); break;
+        case 6: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_faces_fp64_batch_kernel<3>, FaceTile<3>::NTHREAD, 0); break;
+        case 7: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dg_cell_fp64_batch_kernel<3>, CellTile<3>::NTHREAD, 0); break;
         default: break;
     }
     return n;
