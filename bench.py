@@ -389,7 +389,7 @@ def measure_single(name: str, args, rank: int, world: int, local: int, pg, e2e: 
                      else DG_MIXED_KERNEL.get(pth["tpc"], "dg_stage_mixed_kernel"))
         if prec == "fp64_fma":
             kname = ("weno_stage_fp64_kernel, FMA-contracted build" if w["method"] == "weno"
-                     else "dg_stage_fused_fp64_kernel (one fused FP64 launch per stage, FMA)")
+                     else "dg_face_kernel + dg_cell_kernel (one stage), FMA-contracted build")
         roofs[prec] = {
             "bound": "fp64" if f64 else "fp32", "achieved": achieved, "peak": pk,
             "unit": "TFLOP/s", "frac": achieved / pk,
@@ -709,7 +709,7 @@ def gpu_launches(w, prec) -> int:
     """Kernels of this library launched per step on the headline path."""
     if w["method"] == "weno":
         return 3
-    per_stage = 1 if prec == "mixed" else 3
+    per_stage = 1 if prec == "mixed" else 2
     lim = (w["opts"].get("fp64" if prec == "fp64_fma" else prec, {}) if "fp64" in w["opts"]
            else w["opts"]).get("limiter", "reference")
     return 3 * (per_stage + (1 if lim in ("tvb", "tvb_mlp") else 0))

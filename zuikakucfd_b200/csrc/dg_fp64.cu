@@ -25,8 +25,8 @@
 #include "zk_internal.h"
 
 // Built twice: with --fmad=false as the reference-arithmetic path (namespace
-// zk), and with -DZK_FP64_FMA, fused multiply-adds contracted, as the
-// ZK_PREC_FP64_FMA path (namespace zk_fma).
+// zk), and with -DZK_FP64_FMA, fused multiply-adds contracted and the cell
+// integrals sum-factorised, as the ZK_PREC_FP64_FMA path (namespace zk_fma).
 #ifdef ZK_FP64_FMA
 #define ZK_FP64_NS zk_fma
 #else
@@ -35,6 +35,12 @@
 
 namespace ZK_FP64_NS {
 using namespace zk;
+
+#ifdef ZK_FP64_FMA
+constexpr bool kFma = true;
+#else
+constexpr bool kFma = false;
+#endif
 
 __constant__ DGTab c_dgtab[3];
 
@@ -380,6 +386,9 @@ struct CellTile {
     double sd[4 * NM][32];      // filled stage input; later the limiter's view of the result
     double fg[CH * NQ][8][32];  // F and G at the round's points; later the limiter's exchange
     double fx[4 * NQ][33], fyu[4 * NQ][32], fyd[4 * NQ][32];  // interface fluxes
+    // mode of thread (lane, w)'s n-th accumulator: px = w in the reference's
+    // summation order, py = w where the sums are factorised
+    static __device__ __forceinline__ int mode(int w, int n) { return kFma ? n * NQ + w : w * NQ + n; }
 };
 
 // applyLimiter (src_DG/fluid.cpp:824-992) on the tile: Persson modal filter
@@ -403,7 +412,7 @@ __device__ __forceinline__ void limit_tile(CellTile<P>& S, double (&o)[4][P + 1]
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int n = 0; n < NQ; ++n) S.sd[c * NM + w * NQ + n][lane] = o[c][n];
+        for (int n = 0; n < NQ; ++n) S.sd[c * NM + CellTile<P>::mode(w, n)][lane] = o[c][n];
     __syncthreads();
     for (int c = w; c < 4; c += NQ) {
         double f = 1.0;
@@ -437,7 +446,7 @@ __device__ __forceinline__ void limit_tile(CellTile<P>& S, double (&o)[4][P + 1]
         for (int n = 0; n < NQ; ++n) {
             if (w == P || n == P) {
                 o[c][n] *= f;
-                S.sd[c * NM + w * NQ + n][lane] = o[c][n];
+                S.sd[c * NM + CellTile<P>::mode(w, n)][lane] = o[c][n];
             }
             if (w < NZ && n < NZ && (w || n)) spread += fabs(o[c][n]);
         }
@@ -484,7 +493,7 @@ __device__ __forceinline__ void limit_tile(CellTile<P>& S, double (&o)[4][P + 1]
                 for (int n = 0; n < NQ; ++n)
                     if (w || n) {
                         o[c][n] *= theta_rho;
-                        S.sd[c * NM + w * NQ + n][lane] = o[c][n];
+                        S.sd[c * NM + CellTile<P>::mode(w, n)][lane] = o[c][n];
                     }
     }
     const double p_avg = (gamma - 1.0) * (E0 - 0.5 * (mx0 * mx0 + my0 * my0) / rho0);
@@ -534,13 +543,231 @@ __device__ __forceinline__ void limit_tile(CellTile<P>& S, double (&o)[4][P + 1]
                 if (w || n) o[c][n] *= theta_p;
 }
 
+// The volume and face integrals of cell `lane` in the reference's order of
+// operations (thread px = w), added to o.
+template <int P>
+__device__ __forceinline__ void integrals(const DGTab& T, CellTile<P>& S, double gamma, double (&o)[4][P + 1]) {
+    constexpr int NQ = P + 1, NM = NQ * NQ, CH = CellTile<P>::CH;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // volume integral (src_DG/fluid.cpp:698-718), CH rows of points at a time
+#pragma unroll 1
+    for (int qa0 = 0; qa0 < NQ; qa0 += CH) {
+        double U[CH][4];
+#pragma unroll
+        for (int u = 0; u < CH; ++u)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) U[u][c] = S.sd[c * NM][lane];  // phi_0 = 1
+#pragma unroll
+        for (int m = 1; m < NM; ++m)
+#pragma unroll
+            for (int u = 0; u < CH; ++u) {
+                const double b = T.vphi[(qa0 + u) * NQ + w][m];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) U[u][c] += S.sd[c * NM + m][lane] * b;
+            }
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+            double F[4], G[4];
+            euler_flux(U[u], gamma, F, G);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                S.fg[u * NQ + w][c][lane] = F[c];
+                S.fg[u * NQ + w][4 + c][lane] = G[c];
+            }
+        }
+        __syncthreads();
+        // terms whose basis derivative is 0 identically (d/dxi at px = 0,
+        // d/deta at py = 0) add +-0 and are left out, but for mode 0, whose
+        // sum still turns NaN on a non-finite flux as the reference's does
+#pragma unroll 1
+        for (int pt = 0; pt < CH * NQ; ++pt) {
+            const int p = qa0 * NQ + pt;
+            const double coeff = T.vw[p];
+            double F[4], G[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                F[c] = S.fg[pt][c][lane];
+                G[c] = S.fg[pt][4 + c][lane];
+            }
+            if (w == 0) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) o[c][0] += coeff * (F[c] * 0.0 + G[c] * 0.0);
+#pragma unroll
+                for (int n = 1; n < NQ; ++n) {
+                    const double det = T.vdet[p][n];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) o[c][n] += coeff * (G[c] * det);
+                }
+            } else {
+                const double dx0 = T.vdxi[p][w * NQ];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) o[c][0] += coeff * (F[c] * dx0);
+#pragma unroll
+                for (int n = 1; n < NQ; ++n) {
+                    const double dxi = T.vdxi[p][w * NQ + n], det = T.vdet[p][w * NQ + n];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) o[c][n] += coeff * (F[c] * dxi + G[c] * det);
+                }
+            }
+        }
+        if (qa0 + CH < NQ) __syncthreads();
+    }
+    copy_wait<0>();
+    __syncthreads();
+    // face integrals: right (-), left (+), bottom (-), top (+)
+    // (src_DG/fluid.cpp:731-796).  P_n(+1) = 1 and P_n(-1) = (-1)^n exactly,
+    // so an x face's weights are those of px = 0 up to sign, and a y face's
+    // weight is one per thread: its product serves all NQ modes.
+    const bool odd = w & 1;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double f = S.fx[q * 4 + c][lane + 1];
+#pragma unroll
+            for (int n = 0; n < NQ; ++n) o[c][n] -= T.bv[0][q][n] * f;
+        }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double x = S.fx[q * 4 + c][lane], f = odd ? -x : x;
+#pragma unroll
+            for (int n = 0; n < NQ; ++n) o[c][n] += T.bv[0][q][n] * f;
+        }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const double b = T.bv[2][q][w * NQ];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double t = b * S.fyd[q * 4 + c][lane];
+#pragma unroll
+            for (int n = 0; n < NQ; ++n) o[c][n] -= t;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const double b = T.bv[2][q][w * NQ];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double t = b * S.fyu[q * 4 + c][lane];
+#pragma unroll
+            for (int n = 0; n < NQ; ++n) o[c][n] += (n & 1) ? -t : t;
+        }
+    }
+}
+
+// The same integrals by sum factorisation (ZK_PREC_FP64_FMA; thread py = w):
+// phi_m = P_px(xi) P_py(eta), so the state at a point contracts px first (own
+// modes only) and py at the point, and the projection back contracts eta at
+// fixed xi, then xi: 384 multiply-adds per thread at P=3 where the direct sums
+// take 768.  With one fused launch per stage (two threads per cell, tile and
+// interface fluxes in one CTA: 208 registers, 8 warps per SM, FP64 pipe 23%)
+// the P=3 stage at 768^2 took 1,077 us, with this pass and the face pass
+// 598 us.
+template <int P>
+__device__ __forceinline__ void integrals_factored(const DGTab& T, CellTile<P>& S, double gamma,
+                                                   double (&o)[4][P + 1]) {
+    constexpr int NQ = P + 1, NM = NQ * NQ, CH = CellTile<P>::CH;
+    static_assert(NQ * NQ * 4 <= CH * NQ * 8, "the xi-contracted modes fit the flux buffer");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // one-dimensional factors at Gauss point q: P_n, P_n', and P_n w_q
+    auto L = [&](int n, int q) { return T.vphi[q * NQ][n * NQ]; };
+    auto D = [&](int n, int q) { return T.vdxi[q * NQ][n * NQ]; };
+    auto WL = [&](int n, int q) { return T.bv[2][q][n * NQ]; };
+    double(*ex)[32] = S.fg[0];  // [py][qa][c]: own modes contracted over px
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        double v[NQ];
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) v[n] = S.sd[c * NM + n * NQ + w][lane];
+#pragma unroll
+        for (int qa = 0; qa < NQ; ++qa) {
+            double e = v[0];
+#pragma unroll
+            for (int n = 1; n < NQ; ++n) e += v[n] * L(n, qa);
+            ex[(w * NQ + qa) * 4 + c][lane] = e;
+        }
+    }
+    __syncthreads();
+    double U[NQ][4];  // the state at the points (qa, qb = w)
+#pragma unroll
+    for (int qa = 0; qa < NQ; ++qa)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) U[qa][c] = ex[qa * 4 + c][lane];
+#pragma unroll
+    for (int n = 1; n < NQ; ++n) {
+        const double b = L(n, w);
+#pragma unroll
+        for (int qa = 0; qa < NQ; ++qa)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) U[qa][c] += ex[(n * NQ + qa) * 4 + c][lane] * b;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int qa0 = 0; qa0 < NQ; qa0 += CH) {
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+            double F[4], G[4];
+            euler_flux(U[qa0 + u], gamma, F, G);
+            const double coeff = T.vw[(qa0 + u) * NQ + w];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                S.fg[u * NQ + w][c][lane] = F[c] * coeff;
+                S.fg[u * NQ + w][4 + c][lane] = G[c] * coeff;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+            double f[4] = {0.0, 0.0, 0.0, 0.0}, g[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int qb = 0; qb < NQ; ++qb) {
+                const double l = L(w, qb), d = D(w, qb);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    f[c] += S.fg[u * NQ + qb][c][lane] * l;
+                    g[c] += S.fg[u * NQ + qb][4 + c][lane] * d;
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < NQ; ++n)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) o[c][n] += D(n, qa0 + u) * f[c] + L(n, qa0 + u) * g[c];
+        }
+        if (qa0 + CH < NQ) __syncthreads();
+    }
+    copy_wait<0>();
+    __syncthreads();
+    // face integrals: x faces weigh P_py = w's factor (one sum for all px),
+    // y faces P_px's; P_n(+1) = 1, P_n(-1) = (-1)^n
+    const bool odd = w & 1;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        double r = 0.0, l = 0.0, y[NQ];
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) y[n] = 0.0;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const double b = WL(w, q), u = S.fyu[q * 4 + c][lane];
+            r += b * S.fx[q * 4 + c][lane + 1];
+            l += b * S.fx[q * 4 + c][lane];
+            const double t = (odd ? -u : u) - S.fyd[q * 4 + c][lane];
+#pragma unroll
+            for (int n = 0; n < NQ; ++n) y[n] += WL(n, q) * t;
+        }
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) o[c][n] += (((n & 1) ? -l : l) - r) + y[n];
+    }
+}
+
 // Cells (i, j0 .. j0+31).  Returns the thread's max corner wave speed of the
 // fluid cells written when want_lam (computeMaxSpeedDG_omp), else 0.  Ends with
 // every thread past its reads of S, except for a caller's barrier.
 template <int P>
 __device__ __forceinline__ double cell_tile(const DGArgs& a, int j0, int i, CellTile<P>& S) {
     using C = CellTile<P>;
-    constexpr int NQ = C::NQ, NM = C::NM, CH = C::CH;
+    constexpr int NQ = C::NQ, NM = C::NM;
     const DGTab& T = c_dgtab[P - 1];
     const int ny = a.g.ny, nx = a.g.nx;
     const size_t plane = a.g.plane;
@@ -570,7 +797,7 @@ __device__ __forceinline__ double cell_tile(const DGArgs& a, int j0, int i, Cell
         for (int c = 0; c < 4; ++c)
 #pragma unroll
             for (int n = 0; n < NQ; ++n)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(a.un + (size_t)(c * NM + w * NQ + n) * plane + k));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(a.un + (size_t)(c * NM + CellTile<P>::mode(w, n)) * plane + k));
     }
     copy_wait<1>();
     if (r.neg >= 0)  // slip walls: each thread negates what it copied
@@ -584,112 +811,8 @@ __device__ __forceinline__ double cell_tile(const DGArgs& a, int j0, int i, Cell
 #pragma unroll
         for (int n = 0; n < NQ; ++n) o[c][n] = 0.0;
     if (work) {
-        // volume integral (src_DG/fluid.cpp:698-718), CH rows of points at a time
-#pragma unroll 1
-        for (int qa0 = 0; qa0 < NQ; qa0 += CH) {
-            double U[CH][4];
-#pragma unroll
-            for (int u = 0; u < CH; ++u)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) U[u][c] = S.sd[c * NM][lane];  // phi_0 = 1
-#pragma unroll
-            for (int m = 1; m < NM; ++m)
-#pragma unroll
-                for (int u = 0; u < CH; ++u) {
-                    const double b = T.vphi[(qa0 + u) * NQ + w][m];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) U[u][c] += S.sd[c * NM + m][lane] * b;
-                }
-#pragma unroll
-            for (int u = 0; u < CH; ++u) {
-                double F[4], G[4];
-                euler_flux(U[u], a.gamma, F, G);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    S.fg[u * NQ + w][c][lane] = F[c];
-                    S.fg[u * NQ + w][4 + c][lane] = G[c];
-                }
-            }
-            __syncthreads();
-            // terms whose basis derivative is 0 identically (d/dxi at px = 0,
-            // d/deta at py = 0) add +-0 and are left out, but for mode 0, whose
-            // sum still turns NaN on a non-finite flux as the reference's does
-#pragma unroll 1
-            for (int pt = 0; pt < CH * NQ; ++pt) {
-                const int p = qa0 * NQ + pt;
-                const double coeff = T.vw[p];
-                double F[4], G[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    F[c] = S.fg[pt][c][lane];
-                    G[c] = S.fg[pt][4 + c][lane];
-                }
-                if (w == 0) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) o[c][0] += coeff * (F[c] * 0.0 + G[c] * 0.0);
-#pragma unroll
-                    for (int n = 1; n < NQ; ++n) {
-                        const double det = T.vdet[p][n];
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) o[c][n] += coeff * (G[c] * det);
-                    }
-                } else {
-                    const double dx0 = T.vdxi[p][w * NQ];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) o[c][0] += coeff * (F[c] * dx0);
-#pragma unroll
-                    for (int n = 1; n < NQ; ++n) {
-                        const double dxi = T.vdxi[p][w * NQ + n], det = T.vdet[p][w * NQ + n];
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) o[c][n] += coeff * (F[c] * dxi + G[c] * det);
-                    }
-                }
-            }
-            if (qa0 + CH < NQ) __syncthreads();
-        }
-        copy_wait<0>();
-        __syncthreads();
-        // face integrals: right (-), left (+), bottom (-), top (+)
-        // (src_DG/fluid.cpp:731-796).  P_n(+1) = 1 and P_n(-1) = (-1)^n exactly,
-        // so an x face's weights are those of px = 0 up to sign, and a y face's
-        // weight is one per thread: its product serves all NQ modes.
-        const bool odd = w & 1;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const double f = S.fx[q * 4 + c][lane + 1];
-#pragma unroll
-                for (int n = 0; n < NQ; ++n) o[c][n] -= T.bv[0][q][n] * f;
-            }
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const double x = S.fx[q * 4 + c][lane], f = odd ? -x : x;
-#pragma unroll
-                for (int n = 0; n < NQ; ++n) o[c][n] += T.bv[0][q][n] * f;
-            }
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const double b = T.bv[2][q][w * NQ];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const double t = b * S.fyd[q * 4 + c][lane];
-#pragma unroll
-                for (int n = 0; n < NQ; ++n) o[c][n] -= t;
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const double b = T.bv[2][q][w * NQ];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const double t = b * S.fyu[q * 4 + c][lane];
-#pragma unroll
-                for (int n = 0; n < NQ; ++n) o[c][n] += (n & 1) ? -t : t;
-            }
-        }
+        if constexpr (kFma) integrals_factored<P>(T, S, a.gamma, o);
+        else integrals<P>(T, S, a.gamma, o);
         // inverse mass: (2px+1)(2py+1) * 0.5 / h (src_DG/fluid.cpp:800-804)
 #pragma unroll
         for (int n = 0; n < NQ; ++n) {
@@ -704,7 +827,7 @@ __device__ __forceinline__ double cell_tile(const DGArgs& a, int j0, int i, Cell
 #pragma unroll
             for (int c = 0; c < 4; ++c)
 #pragma unroll
-                for (int n = 0; n < NQ; ++n) a.out[(size_t)(c * NM + w * NQ + n) * plane + k] = o[c][n];
+                for (int n = 0; n < NQ; ++n) a.out[(size_t)(c * NM + CellTile<P>::mode(w, n)) * plane + k] = o[c][n];
         return 0.0;
     }
     // Shu-Osher combine with dt applied (src_DG/fluid.cpp:1024-1026, 1036-1038, 1046-1048)
@@ -712,7 +835,7 @@ __device__ __forceinline__ double cell_tile(const DGArgs& a, int j0, int i, Cell
     for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int n = 0; n < NQ; ++n) {
-            const int v = c * NM + w * NQ + n;
+            const int v = c * NM + CellTile<P>::mode(w, n);
             const double dn = a.un[(size_t)v * plane + k];
             const double dd = a.dt * o[c][n];
             const double x = S.sd[v][lane];
@@ -724,9 +847,15 @@ __device__ __forceinline__ double cell_tile(const DGArgs& a, int j0, int i, Cell
         limit_tile<P>(S, o, j >= 3 && j < nx - 3, upd, T, a.gamma, a.s0);
     if (upd && w == 0) {
         uint32_t flags = 0;
+        if constexpr (kFma) {
+            const double rho = o[0][0], mx = o[1][0], my = o[2][0], E = o[3][0];
+            if (!isfinite(rho) || !isfinite(E)) flags |= STATUS_NAN;
+            if (!((a.gamma - 1.0) * (E - 0.5 * (mx * mx + my * my) / rho) > 0.0)) flags |= STATUS_P;
+        } else {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-            if (isnan(o[c][0])) flags |= STATUS_NAN;
+            for (int c = 0; c < 4; ++c)
+                if (isnan(o[c][0])) flags |= STATUS_NAN;
+        }
         if (!(o[0][0] > 0.0)) flags |= STATUS_RHO;
         if (flags) atomicOr(a.status, flags);
     }
@@ -734,14 +863,14 @@ __device__ __forceinline__ double cell_tile(const DGArgs& a, int j0, int i, Cell
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int n = 0; n < NQ; ++n) a.out[(size_t)(c * NM + w * NQ + n) * plane + k] = o[c][n];
+            for (int n = 0; n < NQ; ++n) a.out[(size_t)(c * NM + CellTile<P>::mode(w, n)) * plane + k] = o[c][n];
     if (!a.want_lam) return 0.0;
     // corner q by warp q mod NQ; corner values of the basis are +-1 (reduce_fp64.cu)
     __syncthreads();
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int n = 0; n < NQ; ++n) S.sd[c * NM + w * NQ + n][lane] = o[c][n];
+        for (int n = 0; n < NQ; ++n) S.sd[c * NM + CellTile<P>::mode(w, n)][lane] = o[c][n];
     __syncthreads();
     double umax = 0.0;
     if (j < nx && (a.kind[k] & KIND_FLUID))
@@ -771,6 +900,7 @@ __global__ void __launch_bounds__(CellTile<P>::NTHREAD, cell_ctas(P)) dg_cell_ke
     cell_tile<P>(a, blockIdx.x * 32, blockIdx.y, S);
 }
 
+#ifndef ZK_FP64_FMA  // the batched runner has no FP64_FMA groups
 // Stage-s arguments of batch item `it` (stage s reads U[s-1], writes U[s % 3]).
 __device__ __forceinline__ DGArgs batch_args(const DgItem& it, int stage) {
     const BatchCtl* ctl = it.ctl;
@@ -855,6 +985,8 @@ __global__ void __launch_bounds__(CellTile<P>::NTHREAD, cell_ctas(P)) dg_cell_fp
     }
 }
 
+#endif
+
 // applyLimiter alone, in place on the state (src_DG/fluid.cpp:824-992).
 template <int P>
 __global__ void __launch_bounds__(CellTile<P>::NTHREAD) dg_limit_kernel(DGArgs a) {
@@ -868,13 +1000,13 @@ __global__ void __launch_bounds__(CellTile<P>::NTHREAD) dg_limit_kernel(DGArgs a
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int n = 0; n < NQ; ++n) o[c][n] = a.out[(size_t)(c * NM + w * NQ + n) * plane + k];
+        for (int n = 0; n < NQ; ++n) o[c][n] = a.out[(size_t)(c * NM + CellTile<P>::mode(w, n)) * plane + k];
     limit_tile<P>(S, o, in, (a.kind[k] & KIND_MASK) == KIND_UPDATED, c_dgtab[P - 1], a.gamma, a.s0);
     if (in)
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int n = 0; n < NQ; ++n) a.out[(size_t)(c * NM + w * NQ + n) * plane + k] = o[c][n];
+            for (int n = 0; n < NQ; ++n) a.out[(size_t)(c * NM + CellTile<P>::mode(w, n)) * plane + k] = o[c][n];
 }
 
 template <int P>
@@ -902,6 +1034,7 @@ cudaError_t launch_dg_stage_fp64(int P, const DGArgs& a, cudaStream_t s) {
     }
 }
 
+#ifndef ZK_FP64_FMA
 // Batch tiles per problem: face pass (ny - 5) ceil(nx/32), cell pass ny ceil(nx/32).
 int dg_fp64_batch_tiles(int pass, int ny, int nx) { return (pass == 0 ? ny - 5 : ny) * ((nx + 31) / 32); }
 
@@ -938,6 +1071,8 @@ int dg_fp64_batch_occupancy(int P, int pass) {
     }
     return n;
 }
+
+#endif
 
 cudaError_t launch_dg_limit_fp64(int P, const DGArgs& a, cudaStream_t s) {
     switch (P) {
