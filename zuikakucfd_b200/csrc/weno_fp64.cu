@@ -7,12 +7,25 @@
 //
 // One CTA owns a 32 x 8 tile of cells.  It stages the tile plus a 3-cell halo
 // of the stage input in shared memory (ghost cells already replaced by their
-// fill source), computes every x and y interface flux of the tile ONCE
-// (the reference computes each interface twice, from both neighbours; both
-// evaluations see the same six inputs in the same order and give the same
-// bits), then forms dU and the Shu-Osher combine for every cell of the tile,
-// ghosts included, exactly as the reference's whole-array Eigen expressions do.
+// fill source), reconstructs both face values of every cell and direction,
+// computes every x and y interface flux of the tile ONCE (the reference
+// computes each interface twice, from both neighbours; both evaluations see
+// the same six inputs in the same order and give the same bits), then forms dU
+// and the Shu-Osher combine for every cell of the tile, ghosts included,
+// exactly as the reference's whole-array Eigen expressions do.
+//
+// Bound: the FP64 pipe.  A cell's smoothness indicators in one direction serve
+// its left-biased value on one face and its right-biased value on the other
+// (the same expressions of the same cells), so the reconstruction runs per
+// cell: 3 indicators, 3 reciprocals and 5 weights where a face evaluates 6, 6
+// and 6; and every division is branch-free (fp64_div.cuh).  About 1,070 FP64
+// instructions per interface become 780: 177 -> 156 us a stage at 1024^2 (FP64
+// pipe 64%; the staging, combine and barrier phases of three CTAs per SM leave
+// the rest).
+#include <atomic>
+
 #include "batch.cuh"
+#include "fp64_div.cuh"
 #include "zk_common.cuh"
 #include "zk_kernels.h"
 
@@ -29,43 +42,72 @@ namespace ZK_FP64_NS {
 using namespace zk;
 namespace {
 
+#ifdef ZK_FP64_FMA
+constexpr bool kExact = false;
+#else
+constexpr bool kExact = true;  // quotients correctly rounded
+#endif
+
 // A tile is 32 x TY cells; NW warps (TY + 1 by default) take the 2 TY + 2
 // face-row tasks (TY + 1 x-face rows, TY + 1 y-face rows) in turn.
 constexpr int TX = 32, HX = TX + 6;
 template <int TY, int NW = TY + 1>
 struct Tile {
-    static constexpr int HY = TY + 6, NWARP = NW, NTHREAD = NW * 32;
+    static constexpr int HY = TY + 6, NTHREAD = NW * 32;
 };
 
-// weno5_reconstruct, src_WENO/fluid.cpp:230-263
-__device__ __forceinline__ void weno5(double UL2, double UL1, double UP, double UR1, double UR2,
-                                      double UR3, double& UL, double& UR) {
-    const double eps = 1e-6, C1 = 13.0 / 12.0, C2 = 0.25;
-    double qL0 = (1.0 / 3.0) * UL2 - (7.0 / 6.0) * UL1 + (11.0 / 6.0) * UP;
-    double qL1 = -(1.0 / 6.0) * UL1 + (5.0 / 6.0) * UP + (1.0 / 3.0) * UR1;
-    double qL2 = (1.0 / 3.0) * UP + (5.0 / 6.0) * UR1 - (1.0 / 6.0) * UR2;
-    double d0 = UL2 - 2 * UL1 + UP, d1 = UL2 - 4 * UL1 + 3 * UP;
-    double d2 = UL1 - 2 * UP + UR1, d3 = UL1 - UR1;
-    double d4 = UP - 2 * UR1 + UR2, d5 = 3 * UP - 4 * UR1 + UR2;
-    double b0 = C1 * d0 * d0 + C2 * d1 * d1, b1 = C1 * d2 * d2 + C2 * d3 * d3,
-           b2 = C1 * d4 * d4 + C2 * d5 * d5;
-    double t0 = eps + b0, t1 = eps + b1, t2 = eps + b2;
-    double a0 = 0.1 / (t0 * t0), a1 = 0.6 / (t1 * t1), a2 = 0.3 / (t2 * t2);
-    double inv = 1.0 / (a0 + a1 + a2);
-    UL = (a0 * qL0 + a1 * qL1 + a2 * qL2) * inv;
-
-    double qR0 = (11.0 / 6.0) * UR1 - (7.0 / 6.0) * UR2 + (1.0 / 3.0) * UR3;
-    double qR1 = (1.0 / 3.0) * UP + (5.0 / 6.0) * UR1 - (1.0 / 6.0) * UR2;
-    double qR2 = -(1.0 / 6.0) * UL1 + (5.0 / 6.0) * UP + (1.0 / 3.0) * UR1;
-    double r0 = UR1 - 2 * UR2 + UR3, r1 = 3 * UR1 - 4 * UR2 + UR3;
-    double r2 = UP - 2 * UR1 + UR2, r3 = UP - UR2;
-    double r4 = UL1 - 2 * UP + UR1, r5 = UL1 - 4 * UP + 3 * UR1;
-    double c0 = C1 * r0 * r0 + C2 * r1 * r1, c1 = C1 * r2 * r2 + C2 * r3 * r3,
-           c2 = C1 * r4 * r4 + C2 * r5 * r5;
-    double s0 = eps + c0, s1 = eps + c1, s2 = eps + c2;
-    double e0 = 0.1 / (s0 * s0), e1 = 0.6 / (s1 * s1), e2 = 0.3 / (s2 * s2);
-    double inv2 = 1.0 / (e0 + e1 + e2);
-    UR = (e0 * qR0 + e1 * qR1 + e2 * qR2) * inv2;
+// weno5_reconstruct, src_WENO/fluid.cpp:230-263, of one cell: from cells
+// i-2 .. i+2 (A B C D E) the left-biased value on its face i+1/2 (UL there)
+// and the right-biased value on its face i-1/2 (UR there).  Products by powers
+// of two are exact, so an explicit fma with one rounds as the reference's
+// separate multiply and add do.
+//
+// PLAIN: every stencil cell's values are plain (see stage_tile), which bounds
+// the squared indicators by 1e-12 and 2^250 and the weights' sums likewise.
+template <bool PLAIN>
+__device__ __forceinline__ void weno5_weights(double t0, double t1, double t2, double (&a)[3], double (&e)[3],
+                                              double& ia, double& ie) {
+    const double q0 = t0 * t0, q1 = t1 * t1, q2 = t2 * t2;
+    if (PLAIN && !ones_low(q0, q1, q2)) {
+        const double y0 = recip<kExact>(q0), y1 = recip<kExact>(q1), y2 = recip<kExact>(q2);
+        a[0] = quot<kExact>(0.1, q0, y0);
+        a[1] = e[1] = quot<kExact>(0.6, q1, y1);
+        a[2] = quot<kExact>(0.3, q2, y2);
+        e[0] = quot<kExact>(0.1, q2, y2);
+        e[2] = quot<kExact>(0.3, q0, y0);
+        const double sa = a[0] + a[1] + a[2], se = e[0] + e[1] + e[2];
+        if (!ones_low(sa, se)) {
+            ia = recip<kExact>(sa);
+            ie = recip<kExact>(se);
+            return;
+        }
+    }
+    a[0] = 0.1 / q0; a[1] = e[1] = 0.6 / q1; a[2] = 0.3 / q2;
+    e[0] = 0.1 / q2; e[2] = 0.3 / q0;
+    ia = 1.0 / (a[0] + a[1] + a[2]);
+    ie = 1.0 / (e[0] + e[1] + e[2]);
+}
+template <bool PLAIN>
+__device__ __forceinline__ void weno5_cell(double A, double B, double C, double D, double E, double& left,
+                                           double& right) {
+    const double eps = 1e-6, C1 = 13.0 / 12.0;
+    const double C3 = 3 * C;
+    const double d0 = __fma_rn(-2.0, B, A) + C, d1 = __fma_rn(-4.0, B, A) + C3;
+    const double d2 = __fma_rn(-2.0, C, B) + D, d3 = B - D;
+    const double d4 = __fma_rn(-2.0, D, C) + E, d5 = __fma_rn(-4.0, D, C3) + E;
+    const double t0 = eps + __fma_rn(0.25, d1 * d1, C1 * d0 * d0);
+    const double t1 = eps + __fma_rn(0.25, d3 * d3, C1 * d2 * d2);
+    const double t2 = eps + __fma_rn(0.25, d5 * d5, C1 * d4 * d4);
+    double a[3], e[3], ia, ie;
+    weno5_weights<PLAIN>(t0, t1, t2, a, e, ia, ie);
+    const double qL0 = (1.0 / 3.0) * A - (7.0 / 6.0) * B + (11.0 / 6.0) * C;
+    const double qL1 = -(1.0 / 6.0) * B + (5.0 / 6.0) * C + (1.0 / 3.0) * D;
+    const double qL2 = (1.0 / 3.0) * C + (5.0 / 6.0) * D - (1.0 / 6.0) * E;
+    left = (a[0] * qL0 + a[1] * qL1 + a[2] * qL2) * ia;
+    const double qR0 = (11.0 / 6.0) * C - (7.0 / 6.0) * D + (1.0 / 3.0) * E;
+    const double qR1 = (1.0 / 3.0) * B + (5.0 / 6.0) * C - (1.0 / 6.0) * D;
+    const double qR2 = -(1.0 / 6.0) * A + (5.0 / 6.0) * B + (1.0 / 3.0) * C;
+    right = (e[0] * qR0 + e[1] * qR1 + e[2] * qR2) * ie;
 }
 
 // muscl_reconstruct, src_WENO/fluid.cpp:203-225 (not called by the reference's
@@ -87,23 +129,25 @@ __device__ __forceinline__ double muscl_slope(double a, double b) {
     }
 }
 template <int LIM>
-__device__ __forceinline__ void muscl(double UL2, double UL1, double UR1, double UR2, double& UL, double& UR) {
-    const double dL = UL1 - UL2, dC = UR1 - UL1, dR = UR2 - UR1;
-    UL = UL1 + 0.5 * muscl_slope<LIM>(dL, dC);
-    UR = UR1 - 0.5 * muscl_slope<LIM>(dC, dR);
+__device__ __forceinline__ void muscl_cell(double B, double C, double D, double& left, double& right) {
+    const double dm = C - B, dp = D - C;
+    left = C + 0.5 * muscl_slope<LIM>(dm, dp);   // UL of face i+1/2: slopes dL, dC
+    right = C - 0.5 * muscl_slope<LIM>(dm, dp);  // UR of face i-1/2: slopes dC, dR
 }
 
-// Face states from the six cells a3 a2 a1 | b1 b2 b3 around a face: WENO5
-// (RECON 0, the reference's scheme) or MUSCL with limiter RECON - 1.
-template <int RECON>
-__device__ __forceinline__ void face_states(double a3, double a2, double a1, double b1, double b2, double b3,
-                                            double& UL, double& UR) {
-    if constexpr (RECON == 0) weno5(a3, a2, a1, b1, b2, b3, UL, UR);
-    else muscl<RECON - 1>(a2, a1, b1, b2, UL, UR);
+// The cell's values on its face i+1/2 (left) and i-1/2 (right): WENO5 (RECON 0,
+// the reference's scheme) or MUSCL with limiter RECON - 1, whose face values
+// depend on the cells i-1, i, i+1 alone.
+template <int RECON, bool PLAIN>
+__device__ __forceinline__ void cell_values(double A, double B, double C, double D, double E, double& left,
+                                            double& right) {
+    if constexpr (RECON == 0) weno5_cell<PLAIN>(A, B, C, D, E, left, right);
+    else muscl_cell<RECON - 1>(B, C, D, left, right);
 }
 
-// hllcFlux (WENO variant), src_WENO/fluid.cpp:268-317
-__device__ __forceinline__ void hllc(const double L[4], const double R[4], double gamma, double F[4]) {
+// hllcFlux (WENO variant), src_WENO/fluid.cpp:268-317, with plain divisions:
+// for operands outside fp64_div.cuh's ranges.
+__device__ __noinline__ void hllc_any(const double* L, const double* R, double gamma, double* F) {
     const double eps = 1e-12;
     double rhoL = ref_max(L[0], eps), uL = L[1] / rhoL, vL = L[2] / rhoL, EL = L[3] / rhoL;
     double pL = ref_max((gamma - 1.0) * (L[3] - 0.5 * rhoL * (uL * uL + vL * vL)), eps);
@@ -145,6 +189,69 @@ __device__ __forceinline__ void hllc(const double L[4], const double R[4], doubl
     F[3] = F3 + S * (s3 - Us[3]);
 }
 
+// The same flux for plain tiles: the same values formed in the same order,
+// quotients over a common denominator sharing its reciprocal.  Plain cells
+// reconstruct to values below 2^63 that are 0 or above 2^-620, so every
+// quotient and remainder below is normal unless a difference underflows or
+// vanishes: den2, r and d are tested.
+__device__ __forceinline__ void hllc_plain(const double (&L)[4], const double (&R)[4], double gamma, double (&F)[4]) {
+    constexpr bool X = kExact;
+    const double eps = 1e-12;
+    const double rhoL = ref_max(L[0], eps), rhoR = ref_max(R[0], eps);
+    const double sqL = sqrt(rhoL), sqR = sqrt(rhoR), den = sqL + sqR;
+    bool ok = !ones_low(rhoL, rhoR, den);
+    {
+        const double yL = recip<X>(rhoL), yR = recip<X>(rhoR);
+        const double uL = quot<X>(L[1], rhoL, yL), vL = quot<X>(L[2], rhoL, yL), EL = quot<X>(L[3], rhoL, yL);
+        const double pL = ref_max((gamma - 1.0) * (L[3] - 0.5 * rhoL * (uL * uL + vL * vL)), eps);
+        const double aL = sqrt(quot<X>(gamma * pL, rhoL, yL));
+        const double uR = quot<X>(R[1], rhoR, yR), vR = quot<X>(R[2], rhoR, yR), ER = quot<X>(R[3], rhoR, yR);
+        const double pR = ref_max((gamma - 1.0) * (R[3] - 0.5 * rhoR * (uR * uR + vR * vR)), eps);
+        const double aR = sqrt(quot<X>(gamma * pR, rhoR, yR));
+        const double yd = recip<X>(den);
+        const double u_roe = quot<X>(sqL * uL + sqR * uR, den, yd);
+        const double h_roe =
+            quot<X>(sqL * (EL + quot<X>(pL, rhoL, yL)) + sqR * (ER + quot<X>(pR, rhoR, yR)), den, yd);
+        const double c_roe = sqrt(ref_max((gamma - 1.0) * (h_roe - 0.5 * u_roe * u_roe), eps));
+        const double SL = ref_min(uL - aL, u_roe - c_roe);
+        const double SR = ref_max(uR + aR, u_roe + c_roe);
+        if (SL >= 0.0) {
+            F[0] = rhoL * uL; F[1] = rhoL * uL * uL + pL; F[2] = rhoL * uL * vL; F[3] = (L[3] + pL) * uL;
+        } else if (SR <= 0.0) {
+            F[0] = rhoR * uR; F[1] = rhoR * uR * uR + pR; F[2] = rhoR * uR * vR; F[3] = (R[3] + pR) * uR;
+        } else {
+            const double num = pR - pL + rhoL * uL * (SL - uL) - rhoR * uR * (SR - uR);
+            double den2 = rhoL * (SL - uL) - rhoR * (SR - uR);
+            if (fabs(den2) < 1e-12) den2 = (den2 >= 0 ? 1e-12 : -1e-12);
+            const double Ss = divide<X>(num, den2);
+            const bool left = (Ss >= 0.0);
+            const double rho = left ? rhoL : rhoR, u = left ? uL : uR, v = left ? vL : vR;
+            const double E = left ? EL : ER, p = left ? pL : pR, S = left ? SL : SR;
+            const double U0 = left ? L[0] : R[0], U1 = left ? L[1] : R[1], U2 = left ? L[2] : R[2],
+                         U3 = left ? L[3] : R[3];
+            const double r = rho * (S - u), d = S - Ss;
+            ok = ok && in_range(den2) && in_range(r) && in_range(d);
+            const double c = divide<X>(r, d);
+            const double s3 = c * (E + (Ss - u) * (Ss + divide<X>(p, r)));
+            F[0] = rho * u + S * (c - U0);
+            F[1] = rho * u * u + p + S * (c * Ss - U1);
+            F[2] = rho * u * v + S * (c * v - U2);
+            F[3] = (U3 + p) * u + S * (s3 - U3);
+        }
+    }
+    if (!ok) {
+        double l[4], r[4], f[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            l[q] = L[q];
+            r[q] = R[q];
+        }
+        hllc_any(l, r, gamma, f);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) F[q] = f[q];
+    }
+}
+
 struct StageArgs {
     const double* Ucur;  // stage input (ghosts unfilled)
     const double* Un;    // state at the start of the step
@@ -161,25 +268,102 @@ struct StageArgs {
 template <int TY>
 struct Smem {
     double sU[4][TY + 6][HX];
-    double sFx[4][TY][TX + 1];
-    double sFy[4][TY + 1][TX];
+    // states left and right of each x / y face; the flux replaces the left one
+    double xl[4][TY][TX + 1], xr[4][TY][TX + 1];
+    double yl[4][TY + 1][TX], yr[4][TY + 1][TX];
     int8_t sK[TY + 6][HX];
 };
+
+// The interface fluxes of a staged tile, each computed once, left in S.xl and
+// S.yl.  First both face values of every cell beside a face, one variable of a
+// row of cells per warp task: TY x rows (columns 0 .. 31), the columns -1 and
+// 32 of all x rows, TY + 2 y rows (rows -1 .. TY); then the fluxes, a row of
+// faces per warp task.
+template <int TY, int NW, int RECON, bool PLAIN>
+__device__ __forceinline__ void tile_fluxes(Smem<TY>& S, double gamma, bool edge) {
+    auto& sU = S.sU;
+    auto& sK = S.sK;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int task = warp; task < 4 * (2 * TY + 3); task += NW) {
+        const int q = task & 3, row = task >> 2;
+        double left, right;
+        if (row <= TY) {
+            int r = row, c = lane;
+            if (row == TY) {
+                if (lane >= 2 * TY) continue;
+                r = lane >> 1;
+                c = (lane & 1) ? TX : -1;
+            }
+            if (edge) {
+                const int8_t* k = &sK[r + 3][c + 3];
+                if (k[-1] != KIND_UPDATED && k[0] != KIND_UPDATED && k[1] != KIND_UPDATED) continue;
+            }
+            const double* u = &sU[q][r + 3][c + 3];
+            cell_values<RECON, PLAIN>(u[-2], u[-1], u[0], u[1], u[2], left, right);
+            if (c < TX) S.xl[q][r][c + 1] = left;
+            if (c >= 0) S.xr[q][r][c] = right;
+        } else {
+            const int r = row - TY - 2, c = lane;
+            if (edge) {
+                const int8_t* k = &sK[r + 3][c + 3];
+                if (k[-HX] != KIND_UPDATED && k[0] != KIND_UPDATED && k[HX] != KIND_UPDATED) continue;
+            }
+            const double* u = &sU[q][r + 3][c + 3];
+            cell_values<RECON, PLAIN>(u[-2 * HX], u[-HX], u[0], u[HX], u[2 * HX], left, right);
+            if (r < TY) S.yl[q][r + 1][c] = left;
+            if (r >= 0) S.yr[q][r][c] = right;
+        }
+    }
+    __syncthreads();
+    for (int task = warp; task < 2 * TY + 2; task += NW) {
+        if (task <= TY) {
+            // x face on the left of tile cell (r, c)
+            int r, c;
+            if (task < TY) { r = task; c = lane; }
+            else { if (lane >= TY) continue; r = lane; c = TX; }
+            if (edge && sK[r + 3][c + 2] != KIND_UPDATED && sK[r + 3][c + 3] != KIND_UPDATED) continue;
+            const double L[4] = {S.xl[0][r][c], S.xl[1][r][c], S.xl[2][r][c], S.xl[3][r][c]};
+            const double R[4] = {S.xr[0][r][c], S.xr[1][r][c], S.xr[2][r][c], S.xr[3][r][c]};
+            double F[4];
+            if constexpr (PLAIN) hllc_plain(L, R, gamma, F);
+            else hllc_any(L, R, gamma, F);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) S.xl[q][r][c] = F[q];
+        } else {
+            // y face above tile cell (r, c); normal momentum swapped in
+            const int r = task - TY - 1, c = lane;
+            if (edge && sK[r + 2][c + 3] != KIND_UPDATED && sK[r + 3][c + 3] != KIND_UPDATED) continue;
+            const double L[4] = {S.yl[0][r][c], S.yl[2][r][c], S.yl[1][r][c], S.yl[3][r][c]};
+            const double R[4] = {S.yr[0][r][c], S.yr[2][r][c], S.yr[1][r][c], S.yr[3][r][c]};
+            double F[4];
+            if constexpr (PLAIN) hllc_plain(L, R, gamma, F);
+            else hllc_any(L, R, gamma, F);
+            S.yl[0][r][c] = F[0];
+            S.yl[1][r][c] = F[1];
+            S.yl[2][r][c] = F[2];
+            S.yl[3][r][c] = F[3];
+        }
+    }
+}
 
 // One tile whose top-left cell is (i0, j0).  Ends with every thread past its
 // last shared-memory read, so a persistent caller may reuse S after a barrier.
 // Returns the thread's max wave speed of the cells it wrote (want_lam), else 0.
 template <int TY, int NW = TY + 1, int RECON = 0>
 __device__ __forceinline__ double stage_tile(const StageArgs& a, int j0, int i0, Smem<TY>& S) {
-    constexpr int HY = Tile<TY, NW>::HY, NWARP = Tile<TY, NW>::NWARP, NTHREAD = Tile<TY, NW>::NTHREAD;
+    constexpr int HY = Tile<TY, NW>::HY, NTHREAD = Tile<TY, NW>::NTHREAD;
     auto& sU = S.sU;
-    auto& sFx = S.sFx;
-    auto& sFy = S.sFy;
+    auto& sFx = S.xl;
+    auto& sFy = S.yl;
     auto& sK = S.sK;
     const int ny = a.g.ny, nx = a.g.nx, pitch = a.g.pitch;
     const size_t plane = a.g.plane;
 
-    // 1. tile + halo of the stage input, ghosts replaced by their source
+    // 1. tile + halo of the stage input, ghosts replaced by their source.
+    //    Plain tiles hold |rho| < 2^60 and momenta and energies that are 0 or
+    //    within 2^-200 .. 2^60 (fp64_div.cuh); edge tiles have cells in or
+    //    beside the tile that are not updated, whose faces may not be needed.
+    bool odd = false, border = false;
     for (int t = threadIdx.x; t < HY * HX; t += NTHREAD) {
         const int r = t / HX, c = t - r * HX;
         const int gi = i0 - 3 + r, gj = j0 - 3 + c;
@@ -188,54 +372,30 @@ __device__ __forceinline__ double stage_tile(const StageArgs& a, int j0, int i0,
         if (gi >= 0 && gi < ny && gj >= 0 && gj < nx) {
             const size_t k = (size_t)gi * pitch + gj;
             kd = a.kind[k] & KIND_MASK;
-            const size_t ks = (kd >= KIND_COPY) ? (size_t)a.gsrc[k] : k;
-            v0 = a.Ucur[ks];
-            v1 = a.Ucur[plane + ks];
-            v2 = a.Ucur[2 * plane + ks];
-            v3 = a.Ucur[3 * plane + ks];
+            v0 = a.Ucur[k];  // beside the kind's load; ghosts load again
+            v1 = a.Ucur[plane + k];
+            v2 = a.Ucur[2 * plane + k];
+            v3 = a.Ucur[3 * plane + k];
+            if (kd >= KIND_COPY) {
+                const size_t ks = (size_t)a.gsrc[k];
+                v0 = a.Ucur[ks];
+                v1 = a.Ucur[plane + ks];
+                v2 = a.Ucur[2 * plane + ks];
+                v3 = a.Ucur[3 * plane + ks];
+            }
         }
         sU[0][r][c] = v0; sU[1][r][c] = v1; sU[2][r][c] = v2; sU[3][r][c] = v3;
         sK[r][c] = kd;
+        odd |= !(fabs(v0) < 0x1p60 && plain_value(v1) && plain_value(v2) && plain_value(v3));
+        border |= kd != KIND_UPDATED && r >= 2 && r < TY + 4 && c >= 2 && c < TX + 4;
     }
+    const bool edge = __syncthreads_or(border);
+    if (!__syncthreads_or(odd)) tile_fluxes<TY, NW, RECON, true>(S, a.gamma, edge);
+    else tile_fluxes<TY, NW, RECON, false>(S, a.gamma, edge);
     __syncthreads();
+    const int lane = threadIdx.x & 31;
 
-    // 2. interface fluxes, each computed once
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int task = warp; task < 2 * TY + 2; task += NWARP) {
-        if (task <= TY) {
-            // x face on the left of tile cell (r, c): cells (r, c-3 .. c+2)
-            int r, c;
-            if (task < TY) { r = task; c = lane; }
-            else { if (lane >= TY) continue; r = lane; c = TX; }
-            const bool need = sK[r + 3][c + 2] == KIND_UPDATED || sK[r + 3][c + 3] == KIND_UPDATED;
-            if (!need) continue;
-            double QL[4], QR[4], F[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                face_states<RECON>(sU[q][r + 3][c], sU[q][r + 3][c + 1], sU[q][r + 3][c + 2], sU[q][r + 3][c + 3],
-                                   sU[q][r + 3][c + 4], sU[q][r + 3][c + 5], QL[q], QR[q]);
-            hllc(QL, QR, a.gamma, F);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) sFx[q][r][c] = F[q];
-        } else {
-            // y face above tile cell (r, c): cells (r-3 .. r+2, c); normal momentum swapped in
-            const int r = task - TY - 1, c = lane;
-            const bool need = sK[r + 2][c + 3] == KIND_UPDATED || sK[r + 3][c + 3] == KIND_UPDATED;
-            if (!need) continue;
-            double QL[4], QR[4], F[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                face_states<RECON>(sU[q][r][c + 3], sU[q][r + 1][c + 3], sU[q][r + 2][c + 3], sU[q][r + 3][c + 3],
-                                   sU[q][r + 4][c + 3], sU[q][r + 5][c + 3], QL[q], QR[q]);
-            double L[4] = {QL[0], QL[2], QL[1], QL[3]}, R[4] = {QR[0], QR[2], QR[1], QR[3]};
-            hllc(L, R, a.gamma, F);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) sFy[q][r][c] = F[q];
-        }
-    }
-    __syncthreads();
-
-    // 3. dU and the stage combine for every cell of the tile
+    // 2. dU and the stage combine for every cell of the tile
     uint32_t flags = 0;
     double umax = 0.0;
     for (int t = threadIdx.x; t < TY * TX; t += NTHREAD) {
@@ -282,11 +442,11 @@ __device__ __forceinline__ double stage_tile(const StageArgs& a, int j0, int i0,
     return umax;
 }
 
-// 3 CTAs per SM (72 registers, no spills): +19% over 2 CTAs at 84 registers.
-template <int RECON>
-__global__ void __launch_bounds__(Tile<8>::NTHREAD, 3) weno_stage_fp64_kernel(StageArgs a) {
-    __shared__ Smem<8> S;
-    stage_tile<8, 9, RECON>(a, blockIdx.x * TX, blockIdx.y * 8, S);
+// Tiles of TY rows worked by NW warps, CTAS of them resident per SM.
+template <int RECON, int TY, int NW, int CTAS>
+__global__ void __launch_bounds__(NW * 32, CTAS) weno_stage_fp64_kernel(StageArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    stage_tile<TY, NW, RECON>(a, blockIdx.x * TX, blockIdx.y * TY, *reinterpret_cast<Smem<TY>*>(smem));
 }
 
 // Persistent stage over every listed problem of a batch group: CTA b takes
@@ -299,7 +459,8 @@ template <int V, int TY = weno_variant_rows(V), int NW = weno_variant_warps(V)>
 __global__ void __launch_bounds__(NW * 32, batch_min_blocks(NW * 32, 864, sizeof(Smem<TY>)))
     weno_stage_fp64_batch_kernel(const WenoItem* __restrict__ items, const int* __restrict__ dir, int cap,
                                  int stage) {
-    __shared__ Smem<TY> S;
+    extern __shared__ __align__(16) unsigned char smem[];
+    Smem<TY>& S = *reinterpret_cast<Smem<TY>*>(smem);
     __shared__ StageArgs sa;  // the current tile's problem, kept out of registers
     __shared__ int s_org[3];  // tile origin x, y; 0 when the problem is not stepping
     __shared__ unsigned long long* s_lam;
@@ -332,16 +493,67 @@ __global__ void __launch_bounds__(NW * 32, batch_min_blocks(NW * 32, 864, sizeof
 }  // namespace
 
 namespace {
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device
+// (once per device and kernel; any host thread may launch).
+template <auto kernel>
+cudaError_t allow_smem(size_t bytes) {
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+    return e;
+}
+template <int V>
+constexpr size_t batch_smem() { return sizeof(Smem<weno_variant_rows(V)>); }
 template <int V>
 cudaError_t launch_batch_v(const WenoItem* items, const int* dir, int cap, int stage, int grid, cudaStream_t s) {
-    weno_stage_fp64_batch_kernel<V><<<grid, weno_variant_warps(V) * 32, 0, s>>>(items, dir, cap, stage);
+    const cudaError_t e = allow_smem<weno_stage_fp64_batch_kernel<V>>(batch_smem<V>());
+    if (e != cudaSuccess) return e;
+    weno_stage_fp64_batch_kernel<V><<<grid, weno_variant_warps(V) * 32, batch_smem<V>(), s>>>(items, dir, cap, stage);
     return cudaGetLastError();
 }
 template <int V>
 int occupancy_v() {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, weno_stage_fp64_batch_kernel<V>, weno_variant_warps(V) * 32, 0);
+    if (allow_smem<weno_stage_fp64_batch_kernel<V>>(batch_smem<V>()) != cudaSuccess) return 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, weno_stage_fp64_batch_kernel<V>, weno_variant_warps(V) * 32,
+                                                  batch_smem<V>());
     return n;
+}
+template <int RECON, int TY, int NW, int CTAS>
+cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s) {
+    constexpr auto kernel = weno_stage_fp64_kernel<RECON, TY, NW, CTAS>;
+    const cudaError_t e = allow_smem<weno_stage_fp64_kernel<RECON, TY, NW, CTAS>>(sizeof(Smem<TY>));
+    if (e != cudaSuccess) return e;
+    const dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY);
+    kernel<<<grid, NW * 32, sizeof(Smem<TY>), s>>>(a);
+    return cudaGetLastError();
+}
+
+// Tile height by the number of tiles.  Throughput favours 8 rows (3 CTAs per
+// SM at 72 registers): a 4- or 2-row tile recomputes more halo values per
+// cell (1024^2: 512 us a step with 8 rows, 574 with 4, 734 with 2, 637 with
+// 16).  But one tile takes about 12, 8 and 6 us with 8, 4 and 2 rows however
+// idle the chip, so a grid whose smaller tiles are all resident at once, two
+// per SM, takes those (64^2 step with its wave speed: 73, 60, 53 us); and
+// where 8-row tiles are too many for one per SM but 16-row tiles are not, the
+// larger tile spares the doubly loaded SMs (256^2: 16.7 -> 15.4 us a stage).
+// One row of 8 x 32 tiles for every size took 13.3 us a stage from 64^2 to
+// 192^2; these take 6.2 (64^2), 7.6 (128^2) and 11.5 us (192^2).
+template <int RECON>
+cudaError_t launch_stage(const StageArgs& a, cudaStream_t s) {
+    constexpr int kSms = 148;
+    if constexpr (RECON == 0) {
+        const long long cols = (a.g.nx + TX - 1) / TX;
+        auto tiles = [&](int rows) { return cols * ((a.g.ny + rows - 1) / rows); };
+        if (tiles(2) <= 2 * kSms) return launch_tiles<RECON, 2, 14, 2>(a, s);
+        if (tiles(4) <= 2 * kSms) return launch_tiles<RECON, 4, 11, 2>(a, s);
+        if (tiles(8) > kSms && tiles(16) <= kSms) return launch_tiles<RECON, 16, 17, 1>(a, s);
+    }
+    return launch_tiles<RECON, 8, 9, 3>(a, s);
 }
 }  // namespace
 
@@ -376,15 +588,13 @@ cudaError_t launch_weno_stage_fp64(const double* Ucur, const double* Un, double*
                                    double dtdx, double dtdy, double gamma, int stage,
                                    uint32_t* status, cudaStream_t s, int recon) {
     StageArgs a{Ucur, Un, Uout, kind, gsrc, g, dtdx, dtdy, gamma, stage, status};
-    dim3 grid((g.nx + TX - 1) / TX, (g.ny + 7) / 8);
     switch (recon) {
-        case 0: weno_stage_fp64_kernel<0><<<grid, Tile<8>::NTHREAD, 0, s>>>(a); break;
-        case 1: weno_stage_fp64_kernel<1><<<grid, Tile<8>::NTHREAD, 0, s>>>(a); break;
-        case 2: weno_stage_fp64_kernel<2><<<grid, Tile<8>::NTHREAD, 0, s>>>(a); break;
-        case 3: weno_stage_fp64_kernel<3><<<grid, Tile<8>::NTHREAD, 0, s>>>(a); break;
+        case 0: return launch_stage<0>(a, s);
+        case 1: return launch_stage<1>(a, s);
+        case 2: return launch_stage<2>(a, s);
+        case 3: return launch_stage<3>(a, s);
         default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 }  // namespace ZK_FP64_NS
