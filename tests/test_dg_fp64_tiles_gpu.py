@@ -86,3 +86,26 @@ def test_nan_spreads_as_in_the_oracle(restatement, P):
     assert word & 1
     assert np.array_equal(np.isfinite(out), np.isfinite(ref))
     assert np.array_equal(out[np.isfinite(ref)], ref[np.isfinite(ref)])
+
+
+@pytest.mark.parametrize("P", [1, 2, 3])
+@pytest.mark.parametrize("kind", ["huge", "tiny", "rest"])
+def test_operands_outside_the_branch_free_division(restatement, P, kind):
+    """Values beyond the shared-reciprocal range next to ordinary ones, and a
+    gas at rest (zero momenta): both divisions round alike."""
+    c, d, b = problem(P, 12, 70, True, 10)
+    r = np.random.default_rng(11)
+    if kind == "huge":
+        d[:, :, :, 35:] *= 2.0 ** 110
+    elif kind == "tiny":
+        d[1:3] = r.choice([0.0, -0.0, 5e-324, 1e-310, 1e-120, 1e-95, -1e-90, 1e-20], size=d[1:3].shape)
+    else:
+        d[1:3] = 0.0
+        d[:, 1:] = 0.0
+    dt = 1e-3 * c.da
+    with open_solver(P, c, b, limiter="none") as s:
+        s.set_state(d)
+        s.step(dt, 1)
+        out = s.get_state()
+    ref = restatement.dg_step_lim(P, d.copy(), b, c.da, c.gamma, dt, 1, limiter="none")
+    assert np.array_equal(out, ref, equal_nan=True)

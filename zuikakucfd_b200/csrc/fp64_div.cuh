@@ -4,9 +4,10 @@
 // carries a range test and a call on its slow path each time, so consecutive
 // divisions cannot overlap, and every division starts from its own
 // reciprocal.  Here the caller vouches for the operands' ranges -- tested once
-// for a whole tile of cells (plain_value), plus a test of the few denominators
-// that differences form (in_range) -- and takes plain `/` elsewhere; inside
-// the range the quotients are straight-line code.
+// for a whole tile of cells (plain_value) or for a state's four values (num_ok),
+// plus a test of the few denominators that differences form (in_range) -- and
+// takes plain `/` elsewhere; inside the range the quotients are straight-line
+// code.
 //
 // Reference-arithmetic build: quotients are correctly rounded, hence bit for
 // bit those of `/`.  With y = RN(1/b) and q within one ulp of a/b,
@@ -32,6 +33,14 @@ namespace zk {
 // word alone, the all-ones significand).
 __device__ __forceinline__ bool in_range(double x) {
     return (uint32_t)((__double2hiint(x) & 0x7fffffff) - 0x20b00000) < 0x3e800000u && __double2loint(x) != -1;
+}
+
+// a == +0 (the quotient of a -0 would lose its sign) or |a| in [2^-300, 2^100):
+// conserved values whose quotients by a density in [1e-5, 2^100), and the
+// fluxes' second-level quotients of those, stay above 2^-800 and below 2^700.
+__device__ __forceinline__ bool num_ok(double a) {
+    const int h = __double2hiint(a);
+    return (uint32_t)((h & 0x7fffffff) - 0x2d300000) < 0x19000000u || (h | __double2loint(a)) == 0;
 }
 
 // Whether any of the values has a low word of all ones: the test that in_range
