@@ -48,7 +48,7 @@ int dg_mixed_batch_tiles(int variant, int ny, int nx);
 int dg_upload_tables_f32(int P);
 int batch_red_tiles(int ny, int nx);
 cudaError_t launch_batch_max_speed(int method, const void* items, const int* dir, int cap, int grid, cudaStream_t s);
-cudaError_t launch_batch_ctl(int post, BatchCtl* ctl, const int* members, int n, const int* admitted,
+cudaError_t launch_batch_ctl(bool post, bool pre, BatchCtl* ctl, const int* members, int n, const int* admitted,
                              cudaStream_t s);
 cudaError_t launch_batch_clock(unsigned long long* t, cudaStream_t s);
 }  // namespace zk
@@ -87,7 +87,6 @@ struct BProblem {
     int xpitch = 0;
     int8_t* kind = nullptr;
     int32_t* gsrc = nullptr;
-    double* phic = nullptr;
     double s0 = 0.0;
     size_t updated = 0;  // updated (bctype 0, interior) cells
     int group = -1, slot = -1;
@@ -221,18 +220,27 @@ cudaError_t launch_stage(zk_batch* b, BGroup& g, int stage, int variant, int cta
                                       s);
 }
 
-// One RK step of group g on stream s; returns kernels launched, or -1.
-int enqueue_group_step(zk_batch* b, BGroup& g, cudaStream_t s) {
+// One RK step of group g on stream s, the first and/or last of its graph;
+// returns kernels launched, or -1.  Problems are admitted between graphs only,
+// so past a graph's first step every running problem's wave speed comes from
+// the previous step's stage 3: no reduction pass, and one control launch ends
+// a step and starts the next (8 problems of 128^2 to 512^2: 14 us a step and
+// group in control kernels, now 5).
+int enqueue_group_step(zk_batch* b, BGroup& g, bool first, bool last, cudaStream_t s) {
+    const int members = (int)g.members.size();
     int n = 0;
-    if (launch_batch_max_speed(g.method, g.d_items, g.d_dir[DIR_RED], g.cap, kRedCtasPerSm * b->sms, s) != cudaSuccess)
-        return -1;
-    if (launch_batch_ctl(0, b->d_ctl, g.d_members, (int)g.members.size(), b->d_admitted, s) != cudaSuccess) return -1;
-    n += 2;
+    if (first) {
+        if (launch_batch_max_speed(g.method, g.d_items, g.d_dir[DIR_RED], g.cap, kRedCtasPerSm * b->sms, s) !=
+            cudaSuccess)
+            return -1;
+        if (launch_batch_ctl(false, true, b->d_ctl, g.d_members, members, b->d_admitted, s) != cudaSuccess) return -1;
+        n += 2;
+    }
     for (int st = 1; st <= 3; ++st) {
         if (launch_stage(b, g, st, g.variant, g.ctas, s) != cudaSuccess) return -1;
         n += (g.dg() && !g.mixed()) ? 2 : 1;
     }
-    if (launch_batch_ctl(1, b->d_ctl, g.d_members, (int)g.members.size(), nullptr, s) != cudaSuccess) return -1;
+    if (launch_batch_ctl(true, !last, b->d_ctl, g.d_members, members, b->d_admitted, s) != cudaSuccess) return -1;
     return n + 1;
 }
 
@@ -281,7 +289,7 @@ int autotune(zk_batch* b, BGroup& g) {
         g.variant = keep;
         if (rc) return rc;
         BK_CUDA(launch_batch_max_speed(g.method, g.d_items, g.d_dir[DIR_RED], g.cap, kRedCtasPerSm * b->sms, b->stream));
-        BK_CUDA(launch_batch_ctl(0, b->d_ctl, g.d_members, (int)g.members.size(), b->d_admitted, b->stream));
+        BK_CUDA(launch_batch_ctl(false, true, b->d_ctl, g.d_members, (int)g.members.size(), b->d_admitted, b->stream));
         int occ = occupancy(g, var);
         if (fp64dg) occ = std::min(occ, dg_fp64_batch_occupancy(g.order, 1));
         for (int c = 1; c <= occ; ++c) {
@@ -323,7 +331,7 @@ int capture(zk_batch* b) {
     for (BGroup& g : b->groups) {
         ok = ok && cudaStreamWaitEvent(g.stream, b->fork, 0) == cudaSuccess;
         for (int s = 0; ok && s < b->opt.graph_steps; ++s) {
-            const int k = enqueue_group_step(b, g, g.stream);
+            const int k = enqueue_group_step(b, g, s == 0, s == b->opt.graph_steps - 1, g.stream);
             ok = k >= 0;
             n += k;
         }
@@ -453,7 +461,6 @@ int finalize(zk_batch* b) {
                 it.fy = p.fy;
                 it.kind = p.kind;
                 it.gsrc = p.gsrc;
-                it.phic = p.phic;
                 it.ctl = b->d_ctl + id;
                 it.g = p.g;
                 it.xpitch = p.xpitch;
@@ -602,13 +609,10 @@ int zk_batch_add(zk_batch* b, const zk_options* o, int ny, int nx, double da, do
         }
     if (dg) {
         DGTab tab;
-        double phic[DG_MAXNM * 4];
-        dg_make_tables(P, &tab, phic);
+        dg_make_tables(P, &tab);
         if (dg_upload_tables(P, tab) != ZK_OK) return bfail(ZK_ERR_CUDA, "DG table upload failed");
         if (mixed && dg_upload_tables_f32(P) != ZK_OK) return bfail(ZK_ERR_CUDA, "DG FP32 table upload failed");
         p.s0 = (P >= 3) ? -3.0 * std::log10((double)P) : -4.0 * std::log10((double)P);
-        if (int rc = balloc_t(b, &p.phic, (size_t)p.nm * 4)) return rc;
-        BK_CUDA(cudaMemcpyAsync(p.phic, phic, sizeof(double) * p.nm * 4, cudaMemcpyHostToDevice, s));
         if (mixed) {
             for (int k = 0; k < 2; ++k) {
                 if (int rc = balloc_t(b, &p.F[k], nvar * p.g.plane)) return rc;
@@ -619,7 +623,6 @@ int zk_batch_add(zk_batch* b, const zk_options* o, int ny, int nx, double da, do
             if (int rc = balloc_t(b, &p.fx, (size_t)NQ * 4 * ny * p.xpitch)) return rc;
             if (int rc = balloc_t(b, &p.fy, (size_t)NQ * 4 * (ny + 1) * p.g.pitch)) return rc;
         }
-        BK_CUDA(cudaStreamSynchronize(s));  // phic is a stack array
     }
     BK_CUDA(cudaStreamSynchronize(s));
     *id = (int)b->probs.size();

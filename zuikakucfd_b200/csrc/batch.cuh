@@ -94,7 +94,6 @@ struct DgItem {
     double* fy;
     const int8_t* kind;
     const int32_t* gsrc;
-    const double* phic;  // basis at the 4 cell corners [NM][4] (CFL reduction)
     BatchCtl* ctl;
     Grid g;
     int xpitch, nm;
@@ -146,6 +145,14 @@ __device__ __forceinline__ double dg_state_speed(const double (&U)[4], double ga
     const double p = ref_max(__dmul_rn(__dsub_rn(gamma, 1.0), __dsub_rn(U[3], __dmul_rn(__dmul_rn(0.5, rho), q))), eps);
     const double a = __dsqrt_rn(__ddiv_rn(__dmul_rn(gamma, p), rho));
     return ref_max(umax, __dadd_rn(__dsqrt_rn(q), a));
+}
+
+// Whether mode m = px NQ + py is -1 (else +1) at corner q = 0..3, the corners
+// (xi, eta) = (-1,-1), (+1,-1), (-1,+1), (+1,+1): P_n(+1) = 1 and P_n(-1) =
+// (-1)^n exactly.
+template <int NQ>
+__host__ __device__ constexpr bool corner_odd(int m, int q) {
+    return (((q & 1) ? 0 : m / NQ) + ((q & 2) ? 0 : m % NQ)) & 1;
 }
 
 // Largest corner wave speed of one DG cell: U at the corners accumulated over

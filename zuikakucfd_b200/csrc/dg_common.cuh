@@ -33,9 +33,8 @@ struct DGSep {
 };
 void dg_make_sep(int P, DGSep* S);
 
-// Host: tabulate P's basis (and the 4 corner values used by the CFL
-// reduction, phic[m*4+k]); upload to the calling TU's constant bank.
-void dg_make_tables(int P, DGTab* T, double* phic);
+// Host: tabulate P's basis; upload to the calling TU's constant bank.
+void dg_make_tables(int P, DGTab* T);
 int dg_upload_tables(int P, const DGTab& T);
 
 struct DGArgs {
@@ -54,7 +53,6 @@ struct DGArgs {
     int hll;             // 1: HLLE instead of HLLC
     double s0;           // Persson threshold -4 log10 P (P<3) or -3 log10 P, from the host's libm
     uint32_t* status;
-    const double* phic;  // basis at the 4 cell corners [NM][4] (want_lam only)
     int want_lam;        // 1: report the max corner wave speed of the fluid cells written
 };
 

@@ -189,8 +189,7 @@ int zk_dg_setup(zk_ctx* c) {
     DGState* s = new DGState();
     c->dg = s;
     zk::DGTab tab;
-    double phic[zk::DG_MAXNM * 4];
-    zk::dg_make_tables(P, &tab, phic);
+    zk::dg_make_tables(P, &tab);
     if (zk::dg_upload_tables(P, tab) != ZK_OK) return zk_internal_fail(ZK_ERR_CUDA, "DG table upload failed");
     if (c->fma() && zk_fma::dg_upload_tables(P, tab) != ZK_OK)
         return zk_internal_fail(ZK_ERR_CUDA, "DG table upload failed");

@@ -83,7 +83,7 @@ const double kGLWt[5][4] = {{0}, {0},
 
 }  // namespace
 
-void dg_make_tables(int P, DGTab* T, double* phic /* [NM][4] */) {
+void dg_make_tables(int P, DGTab* T) {
     std::memset(T, 0, sizeof(DGTab));
     const int NQ = P + 1, NM = NQ * NQ;
     const double* PT = kGLPt[NQ];
@@ -122,9 +122,6 @@ void dg_make_tables(int P, DGTab* T, double* phic /* [NM][4] */) {
                 const double fb = (py == 0) ? 1.0 : (py == 1) ? y : (py == 2) ? 0.5 * (3.0 * y * y - 1.0) : 0.0;
                 T->zs[a * 4 + b][m] = fa * fb;
             }
-    const double XI[4] = {-1.0, +1.0, -1.0, +1.0}, ETA[4] = {-1.0, -1.0, +1.0, +1.0};
-    for (int m = 0; m < NM; ++m)
-        for (int k = 0; k < 4; ++k) phic[m * 4 + k] = phi2(m, XI[k], ETA[k]);
 }
 
 void dg_make_sep(int P, DGSep* S) {
@@ -962,7 +959,7 @@ __device__ __forceinline__ double cell_tile(const DGArgs& a, int j0, int i, Cell
             double cs[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
             for (int m = 0; m < NM; ++m) {
-                const bool neg = (((q & 1) ? 0 : m / NQ) + ((q & 2) ? 0 : m % NQ)) & 1;
+                const bool neg = corner_odd<NQ>(m, q);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const double x = S.sd[c * NM + m][lane];
@@ -1006,7 +1003,6 @@ __device__ __forceinline__ DGArgs batch_args(const DgItem& it, int stage) {
     a.hll = it.hll;
     a.s0 = it.s0;
     a.status = &it.ctl->status;
-    a.phic = it.phic;
     a.want_lam = stage == 3;
     return a;
 }

@@ -70,7 +70,6 @@ struct MixArgs {
     int stage, limiter, hll;
     float s0;
     uint32_t* status;
-    const double* phic;  // basis at the 4 cell corners [NM][4] (LAM kernels only)
     double gamma64;      // gamma in FP64 (LAM kernels only)
     // learned troubled-cell indicator fused into the stage (MLP kernels only):
     // weights, the list the flagged cells are appended to, its count and capacity
@@ -765,7 +764,7 @@ __device__ __forceinline__ double stage_tile(const MixArgs& a, int j0, int i0, f
                 for (int m = 0; m < NM; ++m) {
                     const double o = out[(size_t)(q * NM + m) * plane + k];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) cq[e] = __dadd_rn(cq[e], __dmul_rn(o, __ldg(a.phic + m * 4 + e)));
+                    for (int e = 0; e < 4; ++e) cq[e] = __dadd_rn(cq[e], corner_odd<NQ>(m, e) ? -o : o);
                 }
 #pragma unroll
                 for (int e = 0; e < 4; ++e) cs[e][q] = cq[e];
@@ -1303,7 +1302,11 @@ __device__ __forceinline__ double stage_tile_pair(const MixArgs& a, int j0, int 
                 }
         }
         if (LAM) {
-            // corner values of this half's variables in the state written (read back)
+            // corner values of this half's variables in the state written (read
+            // back); half h then takes corners 2h and 2h + 1, whose other two
+            // variables the partner sends (each half took all four corners,
+            // with a multiply and a table load per term: stage 3 of the P = 2
+            // batch 240 us, now 210)
             double cs[4][2] = {};
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc)
@@ -1311,18 +1314,17 @@ __device__ __forceinline__ double stage_tile_pair(const MixArgs& a, int j0, int 
                 for (int m = 0; m < NM; ++m) {
                     const double o = out[(size_t)((2 * h + cc) * NM + m) * plane + k];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) cs[e][cc] = __dadd_rn(cs[e][cc], __dmul_rn(o, __ldg(a.phic + m * 4 + e)));
+                    for (int e = 0; e < 4; ++e) cs[e][cc] = __dadd_rn(cs[e][cc], corner_odd<NQ>(m, e) ? -o : o);
                 }
-            double full[4][4];
+            const bool fluid = a.kind[k] & KIND_FLUID;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const double o0 = __shfl_xor_sync(pm, cs[e][0], kPairLane), o1 = __shfl_xor_sync(pm, cs[e][1], kPairLane);
-                full[e][0] = h ? o0 : cs[e][0];
-                full[e][1] = h ? o1 : cs[e][1];
-                full[e][2] = h ? cs[e][0] : o0;
-                full[e][3] = h ? cs[e][1] : o1;
+            for (int e = 0; e < 2; ++e) {
+                const double o0 = __shfl_xor_sync(pm, h ? cs[e][0] : cs[2 + e][0], kPairLane);
+                const double o1 = __shfl_xor_sync(pm, h ? cs[e][1] : cs[2 + e][1], kPairLane);
+                const double c0 = h ? cs[2 + e][0] : cs[e][0], c1 = h ? cs[2 + e][1] : cs[e][1];
+                const double U[4] = {h ? o0 : c0, h ? o1 : c1, h ? c0 : o0, h ? c1 : o1};
+                if (fluid) umax = dg_state_speed(U, a.gamma64, umax);
             }
-            if (a.kind[k] & KIND_FLUID) umax = dg_cell_speed(full, a.gamma64, 0.0);
         }
         const double p0 = __shfl_xor_sync(pm, om[0], kPairLane), p1 = __shfl_xor_sync(pm, om[1], kPairLane);
         if (kd == KIND_UPDATED && h == 0) {
@@ -1436,7 +1438,7 @@ __global__ void __launch_bounds__(MTX * dg_variant_rows(V) * dg_variant_tpc(V), 
                 const void* cur = STAGE == 1 ? (const void*)it.U[0] : (const void*)it.F[STAGE - 2];
                 void* out = STAGE == 3 ? (void*)it.U[0] : (void*)it.F[STAGE - 1];
                 sa = MixArgs{cur, it.U[0], out, it.kind, it.gsrc, it.g, ctl->dt, (float)it.inv2h, (float)it.gamma,
-                             STAGE, it.limiter, it.hll, (float)it.s0, &ctl->status, it.phic, it.gamma};
+                             STAGE, it.limiter, it.hll, (float)it.s0, &ctl->status, it.gamma};
                 s_lam = &ctl->lam;
             }
         }
@@ -1538,8 +1540,7 @@ int dg_upload_tables_f32(int P) {
     std::lock_guard<std::mutex> lock(mu);
     if (done[dev] & (1ull << P)) return ZK_OK;
     DGTab T;
-    double phic[DG_MAXNM * 4];
-    dg_make_tables(P, &T, phic);
+    dg_make_tables(P, &T);
     DGTabF F;
     std::memset(&F, 0, sizeof F);
     const double* src = reinterpret_cast<const double*>(&T);

@@ -103,8 +103,7 @@ __device__ __forceinline__ double dg_corner_speed(const double* __restrict__ dof
             const double x = dof[(size_t)(c * NM + m) * plane + k];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const bool neg = (((q & 1) ? 0 : m / NQ) + ((q & 2) ? 0 : m % NQ)) & 1;
-                cs[q][c] += neg ? -x : x;
+                cs[q][c] += corner_odd<NQ>(m, q) ? -x : x;
             }
         }
     return dg_cell_speed(cs, gamma, umax);
@@ -208,55 +207,59 @@ __global__ void __launch_bounds__(256) max_speed_batch_kernel(const void* __rest
     }
 }
 
-// Start of a step: admitted problems that are not finished take a time step
-// from their CFL rule -- WENO dt = cfl da / lambda (the per-step form of
-// src_WENO/solver.cpp:159-171), DG dt = cfl * dgSafeDt (src_DG/solver.cpp:19-23)
-// -- and reset the speed accumulator.  A non-finite or non-positive dt fails
-// the problem.
-__global__ void batch_ctl_pre_kernel(BatchCtl* ctl, const int* __restrict__ members, int n,
-                                     const int* __restrict__ admitted) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        BatchCtl& c = ctl[members[s]];
-        c.stepping = 0;
-        if (!admitted[members[s]] || c.state >= BATCH_DONE) continue;
-        c.state = BATCH_RUNNING;
-        const double lam = __longlong_as_double((long long)c.lam);
-        c.lam = 0ull;
-        c.lam_ready = 0;
-        double dt;
-        if (c.method == ZK_METHOD_DG) dt = c.cfl * (0.9 / (2.0 * (2 * c.order + 1)) * c.da / ref_max(lam, 1e-7));
-        else dt = c.cfl * c.da / lam;
-        if (!(dt > 0.0) || isinf(dt)) {
-            c.state = BATCH_FAILED;
-            c.status |= STATUS_NAN;
-            c.t_done = global_ns();
-            continue;
-        }
-        c.dt = dt;
-        c.dtdx = dt / c.da;
-        c.dtdy = dt / c.da;
-        c.stepping = 1;
+// End of a step (post): count it, log its dt, finish or fail the problem.
+__device__ __forceinline__ void batch_ctl_post(BatchCtl& c) {
+    if (!c.stepping) return;
+    c.stepping = 0;
+    c.dtlog[c.steps_done] = c.dt;
+    c.steps_done += 1;
+    c.t += c.dt;
+    if (c.status & (STATUS_NAN | STATUS_TIMEOUT)) {
+        c.state = BATCH_FAILED;
+        c.t_done = global_ns();
+    } else if (c.steps_done >= c.steps_target) {
+        c.state = BATCH_DONE;
+        c.t_done = global_ns();
+    } else {
+        c.lam_ready = 1;  // stage 3 left the new state's wave speed in lam
     }
 }
 
-// End of a step: count it, log its dt, finish or fail the problem.
-__global__ void batch_ctl_post_kernel(BatchCtl* ctl, const int* __restrict__ members, int n) {
+// Start of a step (pre): admitted problems that are not finished take a time
+// step from their CFL rule -- WENO dt = cfl da / lambda (the per-step form of
+// src_WENO/solver.cpp:159-171), DG dt = cfl * dgSafeDt (src_DG/solver.cpp:19-23)
+// -- and reset the speed accumulator.  A non-finite or non-positive dt fails
+// the problem.
+__device__ __forceinline__ void batch_ctl_pre(BatchCtl& c, bool admitted) {
+    c.stepping = 0;
+    if (!admitted || c.state >= BATCH_DONE) return;
+    c.state = BATCH_RUNNING;
+    const double lam = __longlong_as_double((long long)c.lam);
+    c.lam = 0ull;
+    c.lam_ready = 0;
+    double dt;
+    if (c.method == ZK_METHOD_DG) dt = c.cfl * (0.9 / (2.0 * (2 * c.order + 1)) * c.da / ref_max(lam, 1e-7));
+    else dt = c.cfl * c.da / lam;
+    if (!(dt > 0.0) || isinf(dt)) {
+        c.state = BATCH_FAILED;
+        c.status |= STATUS_NAN;
+        c.t_done = global_ns();
+        return;
+    }
+    c.dt = dt;
+    c.dtdx = dt / c.da;
+    c.dtdy = dt / c.da;
+    c.stepping = 1;
+}
+
+// One thread per problem of the group: the end of a step and/or the start of
+// the next.
+__global__ void batch_ctl_kernel(BatchCtl* ctl, const int* __restrict__ members, int n,
+                                 const int* __restrict__ admitted, bool post, bool pre) {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        BatchCtl& c = ctl[members[s]];
-        if (!c.stepping) continue;
-        c.stepping = 0;
-        c.dtlog[c.steps_done] = c.dt;
-        c.steps_done += 1;
-        c.t += c.dt;
-        if (c.status & (STATUS_NAN | STATUS_TIMEOUT)) {
-            c.state = BATCH_FAILED;
-            c.t_done = global_ns();
-        } else if (c.steps_done >= c.steps_target) {
-            c.state = BATCH_DONE;
-            c.t_done = global_ns();
-        } else {
-            c.lam_ready = 1;  // stage 3 left the new state's wave speed in lam
-        }
+        const int id = members[s];
+        if (post) batch_ctl_post(ctl[id]);
+        if (pre) batch_ctl_pre(ctl[id], admitted[id]);
     }
 }
 
@@ -319,11 +322,9 @@ cudaError_t launch_batch_max_speed(int method, const void* items, const int* dir
     return cudaGetLastError();
 }
 
-cudaError_t launch_batch_ctl(int post, BatchCtl* ctl, const int* members, int n, const int* admitted,
+cudaError_t launch_batch_ctl(bool post, bool pre, BatchCtl* ctl, const int* members, int n, const int* admitted,
                              cudaStream_t s) {
-    const int grid = (n + 127) / 128;
-    if (post) batch_ctl_post_kernel<<<grid, 128, 0, s>>>(ctl, members, n);
-    else batch_ctl_pre_kernel<<<grid, 128, 0, s>>>(ctl, members, n, admitted);
+    batch_ctl_kernel<<<(n + 127) / 128, 128, 0, s>>>(ctl, members, n, admitted, post, pre);
     return cudaGetLastError();
 }
 
