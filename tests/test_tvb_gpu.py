@@ -177,3 +177,29 @@ def test_tensor_core_inference_matches_fp32_forward():
     zt = z[upd]
     assert np.abs(zt - zr).max() <= 0.05 * max(1.0, np.abs(zr).max())
     assert ((zt > 0) == (zr > 0)).mean() >= 0.995
+
+
+@pytest.mark.parametrize("P", [1, 2, 3])
+@pytest.mark.parametrize("ny,nx", [(7, 7), (9, 34), (10, 35), (12, 70)])
+@pytest.mark.parametrize("kind", ["rough", "flat", "extreme"])
+def test_plain_pass_edges(restatement, P, ny, nx, kind):
+    """The plain TVB pass at widths around its 32-cell segments, bit-equal to
+    the restatement: rough states, cells without slopes (which skip the
+    eigenvectors) among rough ones, and means too large, too small or
+    unphysical for that skip."""
+    from zuikakucfd_b200 import cases
+    c = cases.four_quadrant(nx, seed=5, ny=ny)
+    r = np.random.default_rng(12)
+    d = 0.05 * r.standard_normal((4, (P + 1) ** 2, ny, nx))
+    d[:, 0] = c.conserved() * (1.0 + 0.05 * r.standard_normal((4, ny, nx)))
+    if kind != "rough":
+        d[:, [1, P + 1]] *= r.random((1, 1, ny, nx)) < 0.5
+    if kind == "extreme":
+        d[:, 0] *= r.choice([1.0, 1e14, 1e-14], size=(ny, nx))
+        d[3, 0] *= r.choice([1.0, -1.0, 1e-3], size=(ny, nx))
+    with dg_solver(P, c, "tvb") as s:
+        s.set_state(d)
+        s.limit()
+        out = s.get_state()
+    ref, _ = restatement.dg_limit_tvb(P, d.copy(), c.bctype, c.da, c.gamma, M=50.0)
+    assert np.array_equal(out, ref)

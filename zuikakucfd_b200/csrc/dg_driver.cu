@@ -240,7 +240,7 @@ int zk_dg_after_stage(zk_ctx* c, int stage) {
             w = static_cast<const zk::MlpPacked*>(c->mlp);
         }
         e = zk::launch_dg_tvb(c->opt.order, io.out, io.out64, c->kind, c->gsrc, c->g, c->da, c->gamma, c->opt.tvb_M,
-                              c->d_flags, w, nullptr, c->d_nflag, nullptr, w ? io.in : nullptr, io.in64,
+                              nullptr, w, nullptr, c->d_nflag, nullptr, w ? io.in : nullptr, io.in64,
                               c->mlp_screen, c->stream);
     }
     return e == cudaSuccess ? ZK_OK : cuda_fail(e);
@@ -339,7 +339,7 @@ int zk_dg_limit(zk_ctx* c) {
             w = static_cast<const zk::MlpPacked*>(c->mlp);
         }
         cudaError_t e = zk::launch_dg_tvb(c->opt.order, c->Un, true, c->kind, c->gsrc, c->g, c->da, c->gamma,
-                                          c->opt.tvb_M, c->d_flags, w, nullptr, c->d_nflag, nullptr, nullptr, true,
+                                          c->opt.tvb_M, nullptr, w, nullptr, c->d_nflag, nullptr, nullptr, true,
                                           c->mlp_screen, c->stream);
         return e == cudaSuccess ? ZK_OK : cuda_fail(e);
     }

@@ -298,6 +298,10 @@ __device__ __forceinline__ void tvb_cell(const TvbArgs& a, MlpSmem& S, bool gate
 template <typename T, int P>
 __device__ __forceinline__ void tvb_limit(const TvbArgs& a, size_t k, const T (&ub)[4], const T (&uL)[4],
                                           const T (&uR)[4], const T (&uU)[4], const T (&uD)[4]);
+template <typename T, int P>
+__device__ __forceinline__ void tvb_limit_slopes(const TvbArgs& a, size_t k, const T (&ub)[4], const T (&uL)[4],
+                                                 const T (&uR)[4], const T (&uU)[4], const T (&uD)[4],
+                                                 const T (&ax)[4], const T (&ay)[4]);
 
 // 6 CTAs per SM (80 registers, some spilled): the pass is latency-bound, and
 // the extra resident warps beat the 4 CTAs that 110 registers allowed (+1.9%
@@ -411,13 +415,28 @@ __device__ __forceinline__ void tvb_limit(const TvbArgs& a, size_t k, const T (&
                                           const T (&uR)[4], const T (&uU)[4], const T (&uD)[4]) {
     constexpr int NM = (P + 1) * (P + 1);
     const size_t plane = a.g.plane, vs = (size_t)NM * plane;
-    T* d = static_cast<T*>(a.state);
-    const T mh2 = T(a.M) * T(a.da) * T(a.da);
-    T ax[4], ay[4], dxp[4], dxm[4], dyp[4], dym[4], lx[4], ly[4];
+    const T* d = static_cast<const T*>(a.state);
+    T ax[4], ay[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         ax[c] = d[(size_t)c * vs + (size_t)(P + 1) * plane + k];
         ay[c] = d[(size_t)c * vs + plane + k];
+    }
+    tvb_limit_slopes<T, P>(a, k, ub, uL, uR, uU, uD, ax, ay);
+}
+
+// The same with the cell's linear modes (ax: xi, ay: eta) loaded.
+template <typename T, int P>
+__device__ __forceinline__ void tvb_limit_slopes(const TvbArgs& a, size_t k, const T (&ub)[4], const T (&uL)[4],
+                                                 const T (&uR)[4], const T (&uU)[4], const T (&uD)[4],
+                                                 const T (&ax)[4], const T (&ay)[4]) {
+    constexpr int NM = (P + 1) * (P + 1);
+    const size_t plane = a.g.plane, vs = (size_t)NM * plane;
+    T* d = static_cast<T*>(a.state);
+    const T mh2 = T(a.M) * T(a.da) * T(a.da);
+    T dxp[4], dxm[4], dyp[4], dym[4], lx[4], ly[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
         dxp[c] = uR[c] - ub[c];
         dxm[c] = ub[c] - uL[c];
         dyp[c] = uD[c] - ub[c];  // eta grows with the row index
@@ -437,6 +456,57 @@ __device__ __forceinline__ void tvb_limit(const TvbArgs& a, size_t k, const T (&
         for (int m = 0; m < NM; ++m)
             if (m / (P + 1) + m % (P + 1) > 1) d[(size_t)c * vs + (size_t)m * plane + k] = T(0);
     }
+}
+
+// Whether values of ordinary size make up u, so that its eigenvectors (if
+// physical) are finite: p is then 0 or at least about an ulp of E, and the
+// largest entry, |v|^2 / c^2, stays below 1e29 (FP32) or 1e90 (FP64).
+template <typename T>
+__device__ __forceinline__ bool ordinary(const T u[4]) {
+    const T lo = sizeof(T) == 4 ? T(1e-3) : T(1e-12), hi = sizeof(T) == 4 ? T(1e4) : T(1e12);
+    return u[0] > lo && u[0] < hi && fabs(u[1]) < hi && fabs(u[2]) < hi && u[3] > lo && u[3] < hi;
+}
+
+// Plain TVB limiting of every updated cell (no indicator, no features): the
+// pass after each stage of a TVB context.  Bound: the latency of its loads.  A
+// thread issues all 28 at once -- own mean, neighbour means as if no neighbour
+// were a ghost, slopes -- beside the five kinds, and reloads a ghost
+// neighbour's mean from its source (rare); through the general kernel's chain
+// of kind, source and mean, with its shared memory for the network, the pass
+// took 87 us (FP64, P=2, 1030^2) and 49 (FP32).  A cell whose slopes are all 0
+// is unchanged whatever its neighbours hold (0 <= M h^2) and stops there.  Now
+// 53 and 31 us (FP64 with 4, 5, 6, 8 CTAs per SM: 64, 56, 53, 61; FP32 with 8,
+// 10, 12: 31.4, 30.5, 36).
+template <typename T, int P>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 6 : 10) tvb_plain_kernel(TvbArgs a) {
+    constexpr int NM = (P + 1) * (P + 1);
+    const int j = blockIdx.x * 32 + (threadIdx.x & 31), i = 3 + blockIdx.y * 4 + (threadIdx.x >> 5);
+    if (j < 3 || j >= a.g.nx - 3 || i >= a.g.ny - 3) return;  // updated cells lie inside
+    const size_t pitch = a.g.pitch, k = (size_t)i * pitch + j, plane = a.g.plane, vs = (size_t)NM * plane;
+    const size_t kn[4] = {k - 1, k + 1, k - pitch, k + pitch};
+    const T* d = static_cast<const T*>(a.state);
+    const int8_t kd = a.kind[k];
+    int8_t kk[4];
+    T ub[4], un[4][4], ax[4], ay[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) kk[n] = a.kind[kn[n]];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        ub[c] = d[(size_t)c * vs + k];
+        ax[c] = d[(size_t)c * vs + (size_t)(P + 1) * plane + k];
+        ay[c] = d[(size_t)c * vs + plane + k];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) un[n][c] = d[(size_t)c * vs + kn[n]];
+    }
+    if ((kd & KIND_MASK) != KIND_UPDATED) return;
+    bool flat = ordinary<T>(ub);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) flat = flat && ax[c] == T(0) && ay[c] == T(0);
+    if (flat) return;
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+        if ((kk[n] & KIND_MASK) >= KIND_COPY) nb_mean<T>(d, a.kind, a.gsrc, kn[n], vs, un[n]);
+    tvb_limit_slopes<T, P>(a, k, ub, un[0], un[1], un[2], un[3], ax, ay);
 }
 
 // List mode: the cells the fused indicator of the mixed stage kernel flagged
@@ -475,6 +545,16 @@ cudaError_t launch_list_t(int P, const TvbArgs& a, int grid, cudaStream_t s) {
 
 template <typename T>
 cudaError_t launch_t(int P, const TvbArgs& a, cudaStream_t s) {
+    if (!a.mlp && !a.features && !a.flags) {
+        const dim3 grid((a.g.nx + 31) / 32, (a.g.ny - 6 + 3) / 4);
+        switch (P) {
+            case 1: tvb_plain_kernel<T, 1><<<grid, 128, 0, s>>>(a); break;
+            case 2: tvb_plain_kernel<T, 2><<<grid, 128, 0, s>>>(a); break;
+            case 3: tvb_plain_kernel<T, 3><<<grid, 128, 0, s>>>(a); break;
+            default: return cudaErrorInvalidValue;
+        }
+        return cudaGetLastError();
+    }
     dim3 grid((a.g.nx + 127) / 128, (a.g.ny + kTvbRows - 1) / kTvbRows);
     switch (P) {
         case 1: tvb_kernel<T, 1><<<grid, 128, 0, s>>>(a); break;
