@@ -169,6 +169,9 @@ int zk_create(const zk_options* opt, zk_ctx** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
+    if (e == cudaSuccess)
+        e = cudaHostAlloc(reinterpret_cast<void**>(&c->h_max), sizeof *c->h_max,
+                          cudaHostAllocMapped | cudaHostAllocPortable);
     if (e != cudaSuccess) {
         delete c;
         return fail(ZK_ERR_CUDA, "context setup: %s", cudaGetErrorString(e));
@@ -188,6 +191,7 @@ int zk_destroy(zk_ctx* c) {
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
+    if (c->h_max) cudaFreeHost(c->h_max);
     delete c;
     return ZK_OK;
 }
@@ -228,12 +232,13 @@ int zk_set_mesh(zk_ctx* c, int ny, int nx, double da, double gamma, const int32_
     ZK_CUDA(cudaMalloc(&c->S2, bytes));
     ZK_CUDA(cudaMalloc(&c->kind, kind.size()));
     ZK_CUDA(cudaMalloc(&c->gsrc, src.size() * sizeof(int32_t)));
-    ZK_CUDA(cudaMalloc(&c->d_max, sizeof(unsigned long long)));
+    ZK_CUDA(cudaMalloc(&c->d_max, sizeof(MaxSlot)));
     ZK_CUDA(cudaMalloc(&c->d_status, sizeof(uint32_t)));
     ZK_CUDA(cudaMemsetAsync(c->Un, 0, bytes, c->stream));
     ZK_CUDA(cudaMemsetAsync(c->S1, 0, bytes, c->stream));
     ZK_CUDA(cudaMemsetAsync(c->S2, 0, bytes, c->stream));
     ZK_CUDA(cudaMemsetAsync(c->d_status, 0, sizeof(uint32_t), c->stream));
+    ZK_CUDA(cudaMemsetAsync(c->d_max, 0, sizeof(MaxSlot), c->stream));
     ZK_CUDA(cudaMemcpyAsync(c->kind, kind.data(), kind.size(), cudaMemcpyHostToDevice, c->stream));
     ZK_CUDA(cudaMemcpyAsync(c->gsrc, src.data(), src.size() * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
     if (c->opt.method == ZK_METHOD_DG) {
@@ -475,17 +480,15 @@ int zk_max_speed(zk_ctx* c, double* out) {
     if (int rc = check_ctx(c, true)) return rc;
     if (!out) return fail(ZK_ERR_ARG, "null argument");
     ZK_CUDA(cudaSetDevice(c->opt.device));
+    MaxSlot* slot = static_cast<MaxSlot*>(c->d_max);
     if (c->opt.method == ZK_METHOD_DG) {
-        ZK_CUDA(launch_max_speed_dg(c->Un, c->kind, c->g, c->nm, c->gamma, c->d_max, c->sms, c->stream));
+        ZK_CUDA(launch_max_speed_dg(c->Un, c->kind, c->g, c->nm, c->gamma, slot, c->h_max, c->sms, c->stream));
     } else {
-        ZK_CUDA(launch_max_speed_weno(c->Un, c->g, c->gamma, c->d_max, c->sms, c->stream));
+        ZK_CUDA(launch_max_speed_weno(c->Un, c->g, c->gamma, slot, c->h_max, c->sms, c->stream));
     }
-    unsigned long long bits = 0;
-    ZK_CUDA(cudaMemcpyAsync(&bits, c->d_max, sizeof bits, cudaMemcpyDeviceToHost, c->stream));
     ZK_CUDA(cudaStreamSynchronize(c->stream));
-    double v;
-    std::memcpy(&v, &bits, sizeof v);
-    *out = v;
+    const unsigned long long bits = *static_cast<volatile unsigned long long*>(c->h_max);
+    std::memcpy(out, &bits, sizeof bits);
     return ZK_OK;
 }
 

@@ -28,7 +28,8 @@ struct zk_ctx {
     float* F2 = nullptr;
     int8_t* kind = nullptr;   // per-cell kind byte (zk::KIND_*), pitched
     int32_t* gsrc = nullptr;  // fill source (pitched linear index) of ghost cells
-    unsigned long long* d_max = nullptr;
+    void* d_max = nullptr;  // zk::MaxSlot of the wave-speed reduction
+    unsigned long long* h_max = nullptr;  // its result: page-locked host memory, mapped for the device
     uint32_t* d_status = nullptr;
 
     CUtensorMap tmap[3];  // TMA maps over Un, S1, S2 (mixed WENO path)

@@ -40,10 +40,16 @@ inline cudaError_t launch_weno_stage_f64(bool fma, const double* Ucur, const dou
 
 cudaError_t launch_fill_ghosts(double* U, const int8_t* kind, const int32_t* gsrc, const Grid& g,
                                int nvar, int nm, int sms, cudaStream_t s);
-cudaError_t launch_max_speed_weno(const double* U, const Grid& g, double gamma,
-                                  unsigned long long* out, int sms, cudaStream_t s);
+// Accumulator of a max reduction, zero between reductions.
+struct MaxSlot {
+    unsigned long long max;  // bits of the running max (>= 0)
+    uint32_t ticket;         // CTAs done
+};
+// Max wave speed of the state, its bits stored in `host` (mapped host memory).
+cudaError_t launch_max_speed_weno(const double* U, const Grid& g, double gamma, MaxSlot* slot,
+                                  unsigned long long* host, int sms, cudaStream_t s);
 cudaError_t launch_max_speed_dg(const double* dof, const int8_t* kind, const Grid& g, int nm, double gamma,
-                                unsigned long long* out, int sms, cudaStream_t s);
+                                MaxSlot* slot, unsigned long long* host, int sms, cudaStream_t s);
 cudaError_t launch_recover(const double* U, const Grid& g, int nm, double gamma, double* prim,
                            int sms, cudaStream_t s);
 cudaError_t launch_mach(const double* U, const Grid& g, int nm, double gamma, double* mach, double* speed, int sms,
