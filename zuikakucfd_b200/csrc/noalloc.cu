@@ -27,6 +27,7 @@
 #include <mutex>
 
 #include "zk_common.cuh"
+#include "context_id.h"
 #include "zk_internal.h"
 #include "zk_kernels.h"
 
@@ -94,33 +95,6 @@ __global__ void ghost_map_kernel(const int32_t* bct, zk::Grid g, int8_t* kind, i
     }
 }
 
-// Unique id of the calling thread's current CUDA context (driver entry
-// points cuCtxGetCurrent / cuCtxGetId, looked up through the runtime so the
-// library needs no link-time libcuda); false when there is none yet or the
-// driver lacks them.
-bool current_context_id(unsigned long long* id) {
-    using GetCurrent = CUresult (*)(CUcontext*);
-    using GetId = CUresult (*)(CUcontext, unsigned long long*);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<GetCurrent>(p);
-        p = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<GetId>(p);
-    });
-    if (!get_current || !get_id) return false;
-    CUcontext ctx = nullptr;
-    if (get_current(&ctx) != CUDA_SUCCESS || !ctx) return false;
-    return get_id(ctx, id) == CUDA_SUCCESS;
-}
-
 // Device address of the scratch on the current device.  Set-up: the first
 // call on a device (and the first after that device's context was reset)
 // looks the address up with cudaGetSymbolAddress, with the device current;
@@ -133,7 +107,7 @@ int scratch_address(unsigned char** out) {
     std::lock_guard<std::mutex> lock(g_mu);
     ScratchSlot& slot = g_slot[dev];
     unsigned long long id = 0;
-    if (slot.addr && current_context_id(&id) && id == slot.ctx_id) {
+    if (slot.addr && zk::current_context_id(&id) && id == slot.ctx_id) {
         *out = slot.addr;
         return ZK_OK;
     }
@@ -146,7 +120,7 @@ int scratch_address(unsigned char** out) {
     }
     // the lookup made the device's context current; without an id (old
     // driver) nothing is cached and every call looks the address up again
-    if (current_context_id(&id)) {
+    if (zk::current_context_id(&id)) {
         slot.addr = static_cast<unsigned char*>(p);
         slot.ctx_id = id;
     } else {

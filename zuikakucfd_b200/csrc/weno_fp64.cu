@@ -25,6 +25,7 @@
 #include <atomic>
 
 #include "batch.cuh"
+#include "context_id.h"
 #include "fp64_div.cuh"
 #include "zk_common.cuh"
 #include "zk_kernels.h"
@@ -493,24 +494,36 @@ __global__ void __launch_bounds__(NW * 32, batch_min_blocks(NW * 32, 864, sizeof
 }  // namespace
 
 namespace {
-// Lets `kernel` take `bytes` of dynamic shared memory on the current device
-// (once per device and kernel; any host thread may launch).
 template <auto kernel>
-cudaError_t allow_smem(size_t bytes) {
-    static std::atomic<bool> done[64];
+cudaError_t set_smem(size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+// Runs `set` (kernel attributes) unless it has run in the current device's
+// context; any host thread may launch.  `done`: context id per device.
+template <typename Set>
+cudaError_t once_per_context(std::atomic<unsigned long long> (&done)[64], Set set) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+    unsigned long long id = 0;
+    const bool known = dev >= 0 && dev < 64 && current_context_id(&id);
+    if (known && done[dev].load(std::memory_order_acquire) == id + 1) return cudaSuccess;
+    e = set();
+    // the runtime calls above made the context current if it was not
+    if (e == cudaSuccess && dev >= 0 && dev < 64 && current_context_id(&id))
+        done[dev].store(id + 1, std::memory_order_release);
     return e;
 }
 template <int V>
 constexpr size_t batch_smem() { return sizeof(Smem<weno_variant_rows(V)>); }
 template <int V>
+cudaError_t batch_ready() {
+    static std::atomic<unsigned long long> done[64];
+    return once_per_context(done, [] { return set_smem<weno_stage_fp64_batch_kernel<V>>(batch_smem<V>()); });
+}
+template <int V>
 cudaError_t launch_batch_v(const WenoItem* items, const int* dir, int cap, int stage, int grid, cudaStream_t s) {
-    const cudaError_t e = allow_smem<weno_stage_fp64_batch_kernel<V>>(batch_smem<V>());
+    const cudaError_t e = batch_ready<V>();
     if (e != cudaSuccess) return e;
     weno_stage_fp64_batch_kernel<V><<<grid, weno_variant_warps(V) * 32, batch_smem<V>(), s>>>(items, dir, cap, stage);
     return cudaGetLastError();
@@ -518,18 +531,15 @@ cudaError_t launch_batch_v(const WenoItem* items, const int* dir, int cap, int s
 template <int V>
 int occupancy_v() {
     int n = 0;
-    if (allow_smem<weno_stage_fp64_batch_kernel<V>>(batch_smem<V>()) != cudaSuccess) return 0;
+    if (batch_ready<V>() != cudaSuccess) return 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, weno_stage_fp64_batch_kernel<V>, weno_variant_warps(V) * 32,
                                                   batch_smem<V>());
     return n;
 }
 template <int RECON, int TY, int NW, int CTAS>
 cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s) {
-    constexpr auto kernel = weno_stage_fp64_kernel<RECON, TY, NW, CTAS>;
-    const cudaError_t e = allow_smem<weno_stage_fp64_kernel<RECON, TY, NW, CTAS>>(sizeof(Smem<TY>));
-    if (e != cudaSuccess) return e;
     const dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY);
-    kernel<<<grid, NW * 32, sizeof(Smem<TY>), s>>>(a);
+    weno_stage_fp64_kernel<RECON, TY, NW, CTAS><<<grid, NW * 32, sizeof(Smem<TY>), s>>>(a);
     return cudaGetLastError();
 }
 
@@ -546,6 +556,19 @@ cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s) {
 template <int RECON>
 cudaError_t launch_stage(const StageArgs& a, cudaStream_t s) {
     constexpr int kSms = 148;
+    // every tile height at once: a later call with another grid may be inside a
+    // stream capture, where no kernel should be loaded for the first time
+    static std::atomic<unsigned long long> done[64];
+    const cudaError_t e = once_per_context(done, [] {
+        cudaError_t r = set_smem<weno_stage_fp64_kernel<RECON, 8, 9, 3>>(sizeof(Smem<8>));
+        if constexpr (RECON == 0) {
+            if (r == cudaSuccess) r = set_smem<weno_stage_fp64_kernel<0, 2, 14, 2>>(sizeof(Smem<2>));
+            if (r == cudaSuccess) r = set_smem<weno_stage_fp64_kernel<0, 4, 11, 2>>(sizeof(Smem<4>));
+            if (r == cudaSuccess) r = set_smem<weno_stage_fp64_kernel<0, 16, 17, 1>>(sizeof(Smem<16>));
+        }
+        return r;
+    });
+    if (e != cudaSuccess) return e;
     if constexpr (RECON == 0) {
         const long long cols = (a.g.nx + TX - 1) / TX;
         auto tiles = [&](int rows) { return cols * ((a.g.ny + rows - 1) / rows); };
