@@ -21,6 +21,7 @@
 #include <mutex>
 
 #include "batch.cuh"
+#include "chain.cuh"
 #include "dg_common.cuh"
 #include "fp64_div.cuh"
 #include "zk_internal.h"
@@ -445,6 +446,7 @@ __device__ __forceinline__ void face_tile(const DGArgs& a, int j0, int i, FaceTi
 template <int P>
 __global__ void __launch_bounds__(FaceTile<P>::NTHREAD) dg_face_kernel(DGArgs a) {
     __shared__ FaceTile<P> S;
+    chain_wait();
     face_tile<P>(a, blockIdx.x * 32, 3 + blockIdx.y, S);  // rows 3 .. ny-3 hold every face of an updated cell
 }
 
@@ -978,6 +980,7 @@ constexpr int cell_ctas(int P) { return P == 3 ? 4 : P == 2 ? 6 : 12; }
 template <int P>
 __global__ void __launch_bounds__(CellTile<P>::NTHREAD, cell_ctas(P)) dg_cell_kernel(DGArgs a) {
     __shared__ CellTile<P> S;
+    chain_wait();
     cell_tile<P>(a, blockIdx.x * 32, blockIdx.y, S);
 }
 
@@ -1092,9 +1095,9 @@ __global__ void __launch_bounds__(CellTile<P>::NTHREAD) dg_limit_kernel(DGArgs a
 template <int P>
 cudaError_t launch_stage(const DGArgs& a, cudaStream_t s) {
     const int segs = (a.g.nx + 31) / 32;
-    dg_face_kernel<P><<<dim3(segs, a.g.ny - 5), FaceTile<P>::NTHREAD, 0, s>>>(a);
-    dg_cell_kernel<P><<<dim3(segs, a.g.ny), CellTile<P>::NTHREAD, 0, s>>>(a);
-    return cudaGetLastError();
+    const cudaError_t e = launch_chained(dg_face_kernel<P>, dim3(segs, a.g.ny - 5), FaceTile<P>::NTHREAD, 0, s, a);
+    if (e != cudaSuccess) return e;
+    return launch_chained(dg_cell_kernel<P>, dim3(segs, a.g.ny), CellTile<P>::NTHREAD, 0, s, a);
 }
 
 template <int P>

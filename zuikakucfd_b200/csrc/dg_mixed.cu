@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "batch.cuh"
+#include "chain.cuh"
 #include "dg_common.cuh"
 #include "mlp_infer.cuh"
 #include "zk_internal.h"
@@ -1360,6 +1361,7 @@ constexpr size_t smem_bytes() {
 template <int P, typename TIn, typename TOut>
 __global__ void __launch_bounds__(MTX * 4, P == 1 ? 8 : 3) dg_stage_mixed_kernel(MixArgs a) {
     extern __shared__ __align__(16) float smem[];
+    chain_wait();
     stage_tile<P, TIn, TOut, 4>(a, blockIdx.x * MTX, blockIdx.y * 4, smem);
 }
 
@@ -1391,6 +1393,7 @@ template <int P, typename TIn, typename TOut, bool MLP>
 __global__ void __launch_bounds__(kPairCols * 2 * kPairRows, pair_min_blocks<P, MLP>())
     dg_stage_mixed_pair_kernel(MixArgs a) {
     extern __shared__ __align__(16) float smem[];
+    chain_wait();
     stage_tile_pair<P, TIn, TOut, kPairRows, false, MLP, kPairCols>(a, blockIdx.x * kPairCols, blockIdx.y * kPairRows,
                                                                     smem);
 }
@@ -1510,8 +1513,7 @@ cudaError_t launch_one(const MixArgs& a, cudaStream_t s) {
         attr_set[dev].store(true, std::memory_order_release);
     }
     dim3 grid((a.g.nx + cols - 1) / cols, (a.g.ny + rows - 1) / rows);
-    kern<<<grid, cols * rows * TPC, sm, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(kern, grid, cols * rows * TPC, sm, s, a);
 }
 
 template <int P, typename TIn, typename TOut>

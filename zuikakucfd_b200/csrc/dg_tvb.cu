@@ -16,6 +16,7 @@
 // (tvb_list_kernel) limits only the cells the fused indicator listed.
 #include <cuda_bf16.h>
 
+#include "chain.cuh"
 #include "dg_common.cuh"
 #include "f32x2.cuh"
 #include "zk_internal.h"
@@ -479,6 +480,7 @@ __device__ __forceinline__ bool ordinary(const T u[4]) {
 // 10, 12: 31.4, 30.5, 36).
 template <typename T, int P>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 6 : 10) tvb_plain_kernel(TvbArgs a) {
+    chain_wait();
     constexpr int NM = (P + 1) * (P + 1);
     const int j = blockIdx.x * 32 + (threadIdx.x & 31), i = 3 + blockIdx.y * 4 + (threadIdx.x >> 5);
     if (j < 3 || j >= a.g.nx - 3 || i >= a.g.ny - 3) return;  // updated cells lie inside
@@ -514,6 +516,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 6 : 10) tvb_plain_kernel
 // output; a grid-stride loop over the device-side count.
 template <typename T, int P>
 __global__ void __launch_bounds__(128) tvb_list_kernel(TvbArgs a) {
+    chain_wait();
     constexpr int NM = (P + 1) * (P + 1);
     const size_t vs = (size_t)NM * a.g.plane;
     const T* d = static_cast<const T*>(a.state);
@@ -535,12 +538,11 @@ __global__ void __launch_bounds__(128) tvb_list_kernel(TvbArgs a) {
 template <typename T>
 cudaError_t launch_list_t(int P, const TvbArgs& a, int grid, cudaStream_t s) {
     switch (P) {
-        case 1: tvb_list_kernel<T, 1><<<grid, 128, 0, s>>>(a); break;
-        case 2: tvb_list_kernel<T, 2><<<grid, 128, 0, s>>>(a); break;
-        case 3: tvb_list_kernel<T, 3><<<grid, 128, 0, s>>>(a); break;
+        case 1: return launch_chained(tvb_list_kernel<T, 1>, dim3(grid), 128, 0, s, a);
+        case 2: return launch_chained(tvb_list_kernel<T, 2>, dim3(grid), 128, 0, s, a);
+        case 3: return launch_chained(tvb_list_kernel<T, 3>, dim3(grid), 128, 0, s, a);
         default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 template <typename T>
@@ -548,12 +550,11 @@ cudaError_t launch_t(int P, const TvbArgs& a, cudaStream_t s) {
     if (!a.mlp && !a.features && !a.flags) {
         const dim3 grid((a.g.nx + 31) / 32, (a.g.ny - 6 + 3) / 4);
         switch (P) {
-            case 1: tvb_plain_kernel<T, 1><<<grid, 128, 0, s>>>(a); break;
-            case 2: tvb_plain_kernel<T, 2><<<grid, 128, 0, s>>>(a); break;
-            case 3: tvb_plain_kernel<T, 3><<<grid, 128, 0, s>>>(a); break;
+            case 1: return launch_chained(tvb_plain_kernel<T, 1>, grid, 128, 0, s, a);
+            case 2: return launch_chained(tvb_plain_kernel<T, 2>, grid, 128, 0, s, a);
+            case 3: return launch_chained(tvb_plain_kernel<T, 3>, grid, 128, 0, s, a);
             default: return cudaErrorInvalidValue;
         }
-        return cudaGetLastError();
     }
     dim3 grid((a.g.nx + 127) / 128, (a.g.ny + kTvbRows - 1) / kTvbRows);
     switch (P) {

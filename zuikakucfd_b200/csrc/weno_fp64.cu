@@ -25,6 +25,7 @@
 #include <atomic>
 
 #include "batch.cuh"
+#include "chain.cuh"
 #include "context_id.h"
 #include "fp64_div.cuh"
 #include "zk_common.cuh"
@@ -447,6 +448,7 @@ __device__ __forceinline__ double stage_tile(const StageArgs& a, int j0, int i0,
 template <int RECON, int TY, int NW, int CTAS>
 __global__ void __launch_bounds__(NW * 32, CTAS) weno_stage_fp64_kernel(StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    chain_wait();
     stage_tile<TY, NW, RECON>(a, blockIdx.x * TX, blockIdx.y * TY, *reinterpret_cast<Smem<TY>*>(smem));
 }
 
@@ -539,8 +541,7 @@ int occupancy_v() {
 template <int RECON, int TY, int NW, int CTAS>
 cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s) {
     const dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY);
-    weno_stage_fp64_kernel<RECON, TY, NW, CTAS><<<grid, NW * 32, sizeof(Smem<TY>), s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(weno_stage_fp64_kernel<RECON, TY, NW, CTAS>, grid, NW * 32, sizeof(Smem<TY>), s, a);
 }
 
 // Tile height by the number of tiles.  Throughput favours 8 rows (3 CTAs per

@@ -19,6 +19,7 @@
 // down to a 16-byte boundary) into shared memory; the completion wait is
 // bounded and reports STATUS_TIMEOUT instead of hanging.
 #include "batch.cuh"
+#include "chain.cuh"
 #include "f32x2.cuh"
 #include "tma.cuh"
 #include "tma_host.h"
@@ -399,6 +400,7 @@ __global__ void __launch_bounds__(Tile<8>::NTHREAD, 5)
         mbar_init(&bar, 1);
     }
     __syncthreads();
+    chain_wait();
     double umax;
     stage_tile<8>(&tmap, a, blockIdx.x * TX, blockIdx.y * 8, S, &bar, 0, umax);
 }
@@ -498,8 +500,7 @@ cudaError_t launch_weno_stage_mixed(const CUtensorMap& tmap, const double* Ucur,
                                     double dtdy, double gamma, int stage, uint32_t* status, cudaStream_t s) {
     MixedArgs a{Ucur, Un, Uout, kind, gsrc, g, dtdx, dtdy, gamma, stage, status};
     dim3 grid((g.nx + TX - 1) / TX, (g.ny + 7) / 8);
-    weno_stage_mixed_kernel<<<grid, Tile<8>::NTHREAD, 0, s>>>(tmap, a);
-    return cudaGetLastError();
+    return launch_chained(weno_stage_mixed_kernel, grid, Tile<8>::NTHREAD, 0, s, tmap, a);
 }
 
 // Stage 1 of the mixed WENO step with a barrier that expects 16 bytes more
