@@ -43,7 +43,7 @@ def magnitudes(kind, U, r):
     return U
 
 
-# one ragged size per tile height: 2 rows (the sizes above), 4, 16 and 8
+# one ragged size per tile: 2 rows (the sizes above), 8 rows wide, 16 and 8
 @pytest.mark.parametrize("ny,nx", SIZES + [(97, 201), (173, 301), (241, 517)])
 @pytest.mark.parametrize("kind", ["plain", "huge", "tiny", "vacuum", "nonfinite"])
 def test_weno_step_bits(restatement, ny, nx, kind):

@@ -137,3 +137,25 @@ def test_tma_wait_timeout_is_reported_and_the_context_stays_usable():
     ref, st2 = run(c, dt, 5, "mixed")
     assert st2 == 0
     assert np.array_equal(out, ref)
+
+
+@pytest.mark.parametrize("ny,nx", [(7, 7), (30, 70), (97, 201), (129, 160), (173, 301), (241, 517)])
+@pytest.mark.parametrize("jet", [False, True])
+def test_every_tile_gives_the_same_bits(ny, nx, jet):
+    """The single-problem stage picks its tile by grid size (2 rows, 8 rows
+    wide, 8 rows); each gives the bits of the batch runner's pinned 8-row
+    tile on the same time steps, with FP64 faces (the jet) and without."""
+    from zuikakucfd_b200 import Solver, cases
+    from zuikakucfd_b200.batch import Batch
+    c = cases.high_mach_jet(nx, ny) if jet else cases.four_quadrant(nx, seed=6, ny=ny)
+    U0 = c.conserved()
+    with Batch(policy="all", graph_steps=2, autotune=0, weno_variant=4) as b:
+        pid = b.add(c.bctype, c.da, c.gamma, U0, 3, 0.003 if jet else 0.4, method="weno", precision="mixed")
+        assert b.run()["done"] == 1
+        ref, dts = b.get_state(pid), b.dt_history(pid)
+    with Solver(method="weno", precision="mixed") as s:
+        s.set_mesh(c.ny, c.nx, c.da, c.gamma, c.bctype)
+        s.set_state(U0)
+        for dt in dts:
+            s.step(float(dt), 1)
+        assert np.array_equal(s.get_state(), ref)

@@ -544,16 +544,20 @@ cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s) {
     return launch_chained(weno_stage_fp64_kernel<RECON, TY, NW, CTAS>, grid, NW * 32, sizeof(Smem<TY>), s, a);
 }
 
-// Tile height by the number of tiles.  Throughput favours 8 rows (3 CTAs per
-// SM at 72 registers): a 4- or 2-row tile recomputes more halo values per
-// cell (1024^2: 512 us a step with 8 rows, 574 with 4, 734 with 2, 637 with
-// 16).  But one tile takes about 12, 8 and 6 us with 8, 4 and 2 rows however
-// idle the chip, so a grid whose smaller tiles are all resident at once, two
-// per SM, takes those (64^2 step with its wave speed: 73, 60, 53 us); and
-// where 8-row tiles are too many for one per SM but 16-row tiles are not, the
-// larger tile spares the doubly loaded SMs (256^2: 16.7 -> 15.4 us a stage).
-// One row of 8 x 32 tiles for every size took 13.3 us a stage from 64^2 to
-// 192^2; these take 6.2 (64^2), 7.6 (128^2) and 11.5 us (192^2).
+// Tile by the number of tiles.  Throughput favours 8 rows at 9 warps, 3 CTAs
+// per SM at 72 registers (smaller tiles recompute more halo values per cell,
+// larger ones leave one CTA per SM between its barriers), but a small grid is
+// bound by one tile's latency on a chip mostly idle.  Stage times in us (graph
+// replay; rows/warps x CTAs per SM; tiles of 8 rows):
+//            8/9x3  2/14x2  8/18x1  16/26x1
+//   64^2     13.3     6.3     9.7    14.4       16 tiles
+//   128^2    13.4     7.0     9.8    14.5       64
+//   192^2    13.4    13.0     9.8    14.6      144
+//   256^2    16.7    21.0    17.3    14.6      256
+//   300^2    21.3    28.2    24.5    26.8      380
+//   1024^2  154     313     223     184       4096
+// so the 2-row tile while two per SM are all resident, then one wider tile of
+// 8, then of 16 rows per SM while that suffices, else 8/9.
 template <int RECON>
 cudaError_t launch_stage(const StageArgs& a, cudaStream_t s) {
     constexpr int kSms = 148;
@@ -564,8 +568,8 @@ cudaError_t launch_stage(const StageArgs& a, cudaStream_t s) {
         cudaError_t r = set_smem<weno_stage_fp64_kernel<RECON, 8, 9, 3>>(sizeof(Smem<8>));
         if constexpr (RECON == 0) {
             if (r == cudaSuccess) r = set_smem<weno_stage_fp64_kernel<0, 2, 14, 2>>(sizeof(Smem<2>));
-            if (r == cudaSuccess) r = set_smem<weno_stage_fp64_kernel<0, 4, 11, 2>>(sizeof(Smem<4>));
-            if (r == cudaSuccess) r = set_smem<weno_stage_fp64_kernel<0, 16, 17, 1>>(sizeof(Smem<16>));
+            if (r == cudaSuccess) r = set_smem<weno_stage_fp64_kernel<0, 8, 18, 1>>(sizeof(Smem<8>));
+            if (r == cudaSuccess) r = set_smem<weno_stage_fp64_kernel<0, 16, 26, 1>>(sizeof(Smem<16>));
         }
         return r;
     });
@@ -574,8 +578,8 @@ cudaError_t launch_stage(const StageArgs& a, cudaStream_t s) {
         const long long cols = (a.g.nx + TX - 1) / TX;
         auto tiles = [&](int rows) { return cols * ((a.g.ny + rows - 1) / rows); };
         if (tiles(2) <= 2 * kSms) return launch_tiles<RECON, 2, 14, 2>(a, s);
-        if (tiles(4) <= 2 * kSms) return launch_tiles<RECON, 4, 11, 2>(a, s);
-        if (tiles(8) > kSms && tiles(16) <= kSms) return launch_tiles<RECON, 16, 17, 1>(a, s);
+        if (tiles(8) <= kSms) return launch_tiles<RECON, 8, 18, 1>(a, s);
+        if (tiles(16) <= kSms) return launch_tiles<RECON, 16, 26, 1>(a, s);
     }
     return launch_tiles<RECON, 8, 9, 3>(a, s);
 }

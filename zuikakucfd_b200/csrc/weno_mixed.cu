@@ -387,13 +387,16 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap* tmap, const MixedA
     return true;
 }
 
-// 5 CTAs per SM (40 registers, 384 bytes spilled; 223 KB of shared memory):
-// the extra resident warps hide more latency than the spills cost.  Per step
-// at 2048^2, same bits: 0.618 ms at 5 CTAs, 0.669 ms at 4 (56 registers, 148
-// bytes spilled), 0.765 ms at 3 (72 registers).
-__global__ void __launch_bounds__(Tile<8>::NTHREAD, 5)
+// Tiles of TY rows worked by NW warps, CTAS of them resident per SM (the
+// tensor map's box is that of TY rows).  8 rows: 5 CTAs per SM (40 registers,
+// 384 bytes spilled; 223 KB of shared memory), the extra resident warps hide
+// more latency than the spills cost.  Per step at 2048^2, same bits: 0.618 ms
+// at 5 CTAs, 0.669 ms at 4 (56 registers, 148 bytes spilled), 0.765 ms at 3
+// (72 registers).
+template <int TY, int NW, int CTAS>
+__global__ void __launch_bounds__(NW * 32, CTAS)
     weno_stage_mixed_kernel(const __grid_constant__ CUtensorMap tmap, MixedArgs a) {
-    __shared__ __align__(128) Smem<8> S;
+    __shared__ __align__(128) Smem<TY> S;
     __shared__ __align__(8) uint64_t bar;
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmap);
@@ -402,7 +405,7 @@ __global__ void __launch_bounds__(Tile<8>::NTHREAD, 5)
     __syncthreads();
     chain_wait();
     double umax;
-    stage_tile<8>(&tmap, a, blockIdx.x * TX, blockIdx.y * 8, S, &bar, 0, umax);
+    stage_tile<TY, NW>(&tmap, a, blockIdx.x * TX, blockIdx.y * TY, S, &bar, 0, umax);
 }
 
 // Persistent stage over every listed problem of a batch group (tile variant
@@ -495,12 +498,49 @@ int weno_mixed_batch_occupancy(int variant) {
     }
 }
 
+template <int TY, int NW, int CTAS>
+cudaError_t launch_tiles(const CUtensorMap& tmap, const MixedArgs& a, cudaStream_t s) {
+    const dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY);
+    return launch_chained(weno_stage_mixed_kernel<TY, NW, CTAS>, grid, NW * 32, 0, s, tmap, a);
+}
+
+// Tile of the single-problem stage on a grid.  Throughput favours 8 rows at 9
+// warps, 5 CTAs per SM; a small grid is bound by the latency of one tile, and
+// its chip by idle SMs.  Stage times in us (graph replay; rows/warps; tiles of 8 rows):
+//            8/9    8/18   4/10   2/6
+//   64^2      6.4    5.2    5.1    4.7     16 tiles
+//   128^2     7.1    6.3    6.1    5.5     64
+//   192^2     8.8    6.0    6.6    5.8    144
+//   256^2    11.3    6.9    8.9    9.2    256
+//   300^2    12.3    9.6   10.5   12.1    380
+//   400^2    12.8   14.0   15.6   18.4    650
+//   1024^2   55.3   72.7   86.1  108     4096
+// so 2 rows while those tiles are all resident at four per SM, 18 warps per
+// 8-row tile up to three tiles per SM, else 9.
+enum class MixedTile { Rows2, Rows8Wide, Rows8 };
+static MixedTile mixed_tile(const Grid& g) {
+    constexpr int kSms = 148;
+    const long long cols = (g.nx + TX - 1) / TX;
+    auto tiles = [&](int rows) { return cols * ((g.ny + rows - 1) / rows); };
+    if (tiles(2) <= 4 * kSms) return MixedTile::Rows2;
+    return tiles(8) <= 3 * kSms ? MixedTile::Rows8Wide : MixedTile::Rows8;
+}
+// Box rows of its tensor maps.
+int weno_mixed_rows(const Grid& g) { return mixed_tile(g) == MixedTile::Rows2 ? 2 : 8; }
+
+static cudaError_t launch_grid(const CUtensorMap& tmap, const MixedArgs& a, cudaStream_t s) {
+    switch (mixed_tile(a.g)) {
+        case MixedTile::Rows2: return launch_tiles<2, 6, 4>(tmap, a, s);
+        case MixedTile::Rows8Wide: return launch_tiles<8, 18, 2>(tmap, a, s);
+        default: return launch_tiles<8, 9, 5>(tmap, a, s);
+    }
+}
+
 cudaError_t launch_weno_stage_mixed(const CUtensorMap& tmap, const double* Ucur, const double* Un, double* Uout,
                                     const int8_t* kind, const int32_t* gsrc, const Grid& g, double dtdx,
                                     double dtdy, double gamma, int stage, uint32_t* status, cudaStream_t s) {
     MixedArgs a{Ucur, Un, Uout, kind, gsrc, g, dtdx, dtdy, gamma, stage, status};
-    dim3 grid((g.nx + TX - 1) / TX, (g.ny + 7) / 8);
-    return launch_chained(weno_stage_mixed_kernel, grid, Tile<8>::NTHREAD, 0, s, tmap, a);
+    return launch_grid(tmap, a, s);
 }
 
 // Stage 1 of the mixed WENO step with a barrier that expects 16 bytes more
@@ -511,9 +551,7 @@ cudaError_t launch_weno_timeout_selftest(const CUtensorMap& tmap, const double* 
                                          const int32_t* gsrc, const Grid& g, double dtdx, double dtdy, double gamma,
                                          uint32_t spin, uint32_t* status, cudaStream_t s) {
     MixedArgs a{Un, Un, Uout, kind, gsrc, g, dtdx, dtdy, gamma, 1, status, 0, 16u, spin ? spin : 1u};
-    dim3 grid((g.nx + TX - 1) / TX, (g.ny + 7) / 8);
-    weno_stage_mixed_kernel<<<grid, Tile<8>::NTHREAD, 0, s>>>(tmap, a);
-    return cudaGetLastError();
+    return launch_grid(tmap, a, s);
 }
 
 // Tensor map over one FP64 WENO state: dims (x = nx, y = ny, field = 4),
@@ -532,7 +570,7 @@ int zk_weno_mixed_setup(zk_ctx* c) {
     const char* err = nullptr;
     double* bufs[3] = {c->Un, c->S1, c->S2};
     for (int b = 0; b < 3; ++b)
-        if (!zk::encode_weno_state_map(&c->tmap[b], bufs[b], c->g, &err, 8)) return zk_internal_fail(ZK_ERR_CUDA, err);
+        if (!zk::encode_weno_state_map(&c->tmap[b], bufs[b], c->g, &err, zk::weno_mixed_rows(c->g))) return zk_internal_fail(ZK_ERR_CUDA, err);
     return ZK_OK;
 }
 
