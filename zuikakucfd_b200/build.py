@@ -51,6 +51,7 @@ SOURCES: list[tuple] = [
     ("weno_mixed.cu", ["--use_fast_math"]),
     ("noalloc.cu", []),
     ("slab.cu", []),
+    ("host_copy.cu", []),
     ("batch.cu", []),
 ]
 

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "batch.cuh"
+#include "host_copy.h"
 #include "dg_common.cuh"
 #include "zk_internal.h"
 #include "zuikaku.h"
@@ -125,6 +126,7 @@ struct zk_batch {
     int sms = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, fork = nullptr;
+    HostStage stage;  // staging of large host copies
     std::vector<BProblem> probs;
     std::vector<BGroup> groups;
     BatchCtl* d_ctl = nullptr;
@@ -600,8 +602,7 @@ int zk_batch_add(zk_batch* b, const zk_options* o, int ny, int nx, double da, do
     BK_CUDA(cudaMemcpyAsync(p.gsrc, src.data(), src.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
     if (int rc = balloc(b, reinterpret_cast<void**>(&p.U[0]), bytes)) return rc;
     BK_CUDA(cudaMemsetAsync(p.U[0], 0, bytes, s));
-    BK_CUDA(cudaMemcpy2DAsync(p.U[0], sizeof(double) * p.g.pitch, state, sizeof(double) * nx, sizeof(double) * nx,
-                              nvar * ny, cudaMemcpyHostToDevice, s));
+    BK_CUDA(b->stage.to_device(p.U[0], sizeof(double) * p.g.pitch, state, sizeof(double) * nx, nvar * ny, s));
     if (!(dg && mixed))
         for (int k = 1; k < 3; ++k) {
             if (int rc = balloc(b, reinterpret_cast<void**>(&p.U[k]), bytes)) return rc;
@@ -745,9 +746,8 @@ int zk_batch_get_state(zk_batch* b, int id, double* host) {
     if (id < 0 || id >= (int)b->probs.size()) return bfail(ZK_ERR_ARG, "no problem %d", id);
     const BProblem& p = b->probs[id];
     BK_CUDA(cudaSetDevice(b->opt.device));
-    BK_CUDA(cudaMemcpy2DAsync(host, sizeof(double) * p.nx, p.U[0], sizeof(double) * p.g.pitch, sizeof(double) * p.nx,
-                              (size_t)4 * p.nm * p.ny, cudaMemcpyDeviceToHost, b->stream));
-    BK_CUDA(cudaStreamSynchronize(b->stream));
+    BK_CUDA(b->stage.to_host(host, p.U[0], sizeof(double) * p.g.pitch, sizeof(double) * p.nx, (size_t)4 * p.nm * p.ny,
+                             b->stream));
     return ZK_OK;
 }
 

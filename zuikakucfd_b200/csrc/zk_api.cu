@@ -164,8 +164,7 @@ int zk_create(const zk_options* opt, zk_ctx** out) {
     zk_ctx* c = new zk_ctx();
     c->opt = *opt;
     c->nm = (opt->method == ZK_METHOD_DG) ? (opt->order + 1) * (opt->order + 1) : 1;
-    cudaDeviceProp prop;
-    cudaError_t e = cudaGetDeviceProperties(&prop, opt->device);
+    cudaError_t e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, opt->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
@@ -176,7 +175,6 @@ int zk_create(const zk_options* opt, zk_ctx** out) {
         delete c;
         return fail(ZK_ERR_CUDA, "context setup: %s", cudaGetErrorString(e));
     }
-    c->sms = prop.multiProcessorCount;
     c->stream = c->own_stream;
     *out = c;
     return ZK_OK;
@@ -261,10 +259,8 @@ int zk_set_state(zk_ctx* c, const double* host) {
     if (int rc = check_ctx(c, true)) return rc;
     if (!host) return fail(ZK_ERR_ARG, "null state");
     ZK_CUDA(cudaSetDevice(c->opt.device));
-    ZK_CUDA(cudaMemcpy2DAsync(c->Un, sizeof(double) * c->g.pitch, host, sizeof(double) * c->g.nx,
-                              sizeof(double) * c->g.nx, (size_t)c->nvar * c->g.ny,
-                              cudaMemcpyHostToDevice, c->stream));
-    ZK_CUDA(cudaStreamSynchronize(c->stream));
+    ZK_CUDA(c->stage.to_device(c->Un, sizeof(double) * c->g.pitch, host, sizeof(double) * c->g.nx,
+                               (size_t)c->nvar * c->g.ny, c->stream));
     return ZK_OK;
 }
 
@@ -272,10 +268,8 @@ int zk_get_state(zk_ctx* c, double* host) {
     if (int rc = check_ctx(c, true)) return rc;
     if (!host) return fail(ZK_ERR_ARG, "null state");
     ZK_CUDA(cudaSetDevice(c->opt.device));
-    ZK_CUDA(cudaMemcpy2DAsync(host, sizeof(double) * c->g.nx, c->Un, sizeof(double) * c->g.pitch,
-                              sizeof(double) * c->g.nx, (size_t)c->nvar * c->g.ny,
-                              cudaMemcpyDeviceToHost, c->stream));
-    ZK_CUDA(cudaStreamSynchronize(c->stream));
+    ZK_CUDA(c->stage.to_host(host, c->Un, sizeof(double) * c->g.pitch, sizeof(double) * c->g.nx,
+                             (size_t)c->nvar * c->g.ny, c->stream));
     return ZK_OK;
 }
 
@@ -460,10 +454,8 @@ int zk_rhs(zk_ctx* c, double dt, double* host_dU) {
         const double dtdx = dt / c->da, dtdy = dt / c->da;
         ZK_CUDA(launch_weno_stage_f64(c->fma(), c->Un, c->Un, c->S1, c->kind, c->gsrc, c->g, dtdx, dtdy, c->gamma, 0, c->d_status, c->stream, c->opt.recon));
     }
-    ZK_CUDA(cudaMemcpy2DAsync(host_dU, sizeof(double) * c->g.nx, c->S1, sizeof(double) * c->g.pitch,
-                              sizeof(double) * c->g.nx, (size_t)c->nvar * c->g.ny,
-                              cudaMemcpyDeviceToHost, c->stream));
-    ZK_CUDA(cudaStreamSynchronize(c->stream));
+    ZK_CUDA(c->stage.to_host(host_dU, c->S1, sizeof(double) * c->g.pitch, sizeof(double) * c->g.nx,
+                             (size_t)c->nvar * c->g.ny, c->stream));
     return ZK_OK;
 }
 
@@ -497,10 +489,8 @@ int zk_recover_primitives(zk_ctx* c, double* host_prim) {
     if (!host_prim) return fail(ZK_ERR_ARG, "null argument");
     ZK_CUDA(cudaSetDevice(c->opt.device));
     ZK_CUDA(launch_recover(c->Un, c->g, c->nm, c->gamma, c->S2, c->sms, c->stream));
-    ZK_CUDA(cudaMemcpy2DAsync(host_prim, sizeof(double) * c->g.nx, c->S2, sizeof(double) * c->g.pitch,
-                              sizeof(double) * c->g.nx, (size_t)4 * c->g.ny,
-                              cudaMemcpyDeviceToHost, c->stream));
-    ZK_CUDA(cudaStreamSynchronize(c->stream));
+    ZK_CUDA(c->stage.to_host(host_prim, c->S2, sizeof(double) * c->g.pitch, sizeof(double) * c->g.nx,
+                             (size_t)4 * c->g.ny, c->stream));
     return ZK_OK;
 }
 

@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <vector>
 
+#include "host_copy.h"
 #include "zk_common.cuh"
 #include "zuikaku.h"
 
@@ -31,6 +32,8 @@ struct zk_ctx {
     void* d_max = nullptr;  // zk::MaxSlot of the wave-speed reduction
     unsigned long long* h_max = nullptr;  // its result: page-locked host memory, mapped for the device
     uint32_t* d_status = nullptr;
+
+    zk::HostStage stage;  // staging of large host copies
 
     CUtensorMap tmap[3];  // TMA maps over Un, S1, S2 (mixed WENO path)
 
