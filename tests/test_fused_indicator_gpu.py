@@ -215,3 +215,37 @@ def test_screen_skips_only_cells_near_a_constant_state():
     assert np.array_equal(z1[upd][ev], z0[upd][ev])
     assert np.isneginf(z1[upd][~ev]).all()
     assert n1 == int((z1[upd] > 0).sum()) <= n0
+
+
+@pytest.mark.parametrize("ny,nx", [(8, 16), (9, 17), (15, 33), (25, 15)])
+@pytest.mark.parametrize("P", [2, 3])
+def test_tile_edges(P, ny, nx):
+    """Grids of one 16 x 8 tile, one cell more and one less: with every updated
+    cell listed the step has the plain TVB step's bits, and the screen passes
+    over exactly the cells whose features all lie within it (FP32 features)."""
+    from zuikakucfd_b200 import cases
+    c = cases.four_quadrant(nx, seed=7, ny=ny)
+    dt = dg_dt(P, c)
+    out = {}
+    for lim in ("tvb", "tvb_mlp"):
+        with dg_solver(P, c, lim) as s:
+            if lim == "tvb_mlp":
+                s.set_indicator(constant_logit(1000.0))
+            s.set_state(c.dg_state(P))
+            s.step(dt, 3)
+            out[lim] = s.get_state()
+            if lim == "tvb_mlp":
+                F, z, listed = stage_logits(s, dt, 1)
+                upd = np.zeros((ny, nx), bool)
+                upd[3:-3, 3:-3] = c.bctype[3:-3, 3:-3] == 0
+                tau = float(np.median(np.abs(F).max(axis=1)[upd.ravel()]))
+                assert listed == upd.sum()
+    assert np.array_equal(out["tvb_mlp"], out["tvb"])
+    with dg_solver(P, c, "tvb_mlp") as s:
+        s.set_indicator(constant_logit(1000.0), screen=tau)
+        s.set_state(out["tvb"])
+        F, z, listed = stage_logits(s, dt, 1)
+    dev = np.abs(F).max(axis=1)
+    expect = upd.ravel() & ~(dev <= np.float32(tau))
+    assert np.array_equal(np.isfinite(z) & upd.ravel(), expect)
+    assert listed == expect.sum()

@@ -792,18 +792,17 @@ constexpr int kPairLane = 8;
 __device__ __forceinline__ int pair_half(int t) { return (t >> 3) & 1; }
 __device__ __forceinline__ int pair_cell(int t) { return ((t >> 4) << 3) | (t & 7); }
 
-// Shared memory of the fused indicator: one [16][MLP_TILE_KP] BF16 feature
-// tile per warp (8 warps).  It reuses the interface-flux region, free once
-// every cell has taken its face integrals, where that region is large enough
-// (P = 3), else it follows the stage's own shared memory.  The weights are
-// read through L1 (staging them in shared memory left L1 too small for the
-// stage: measured slower).
-constexpr size_t kMlpTileBytes = 8 * 16 * MLP_TILE_KP * sizeof(uint16_t);
-__host__ __device__ constexpr size_t align16(size_t n) { return (n + 15) & ~size_t(15); }
-template <int P, int MTY, int TX = MTX>
-constexpr bool mlp_tiles_in_flux() {
-    return sizeof(float) * (P + 1) * 4 * (fx_stride(MTY, TX) + fy_stride(MTY, TX)) >= kMlpTileBytes;
-}
+// Feature rows of the fused indicator: 24 words from word kFeatureWord of the
+// cell's own slot of the gathered state.  Once the cell pair has combined, the
+// slot is read again only for the two means the neighbours' features take
+// (words 0 and 3 NM, outside the row), so the rows need no shared memory of
+// their own and no CTA barrier.  With the rows in the interface-flux region
+// (P = 3) or after it (P = 2) behind a CTA barrier, the features formed in every
+// warp and the reference limiter's code in the kernel, the step at 2048^2,
+// four-quadrant, took 5.34 ms (P = 3) and 2.77 ms (P = 2); this form 5.28 and
+// 2.67 ms.  The weights are read through L1 (staging them in shared memory left
+// L1 too small for the stage: measured slower).
+constexpr int kFeatureWord = 1, kFeatureWords = 24;
 
 // Round-to-nearest BF16 pair, lo in the low half.
 __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
@@ -825,43 +824,62 @@ __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
 // every updated, unscreened cell with a positive logit appends the cell to the
 // list, which the TVB list pass then limits.
 template <int P, int TX = MTX>
-__device__ __forceinline__ void indicator_epilogue(const MixArgs& a, const float* sd, uint16_t* ftiles, int slot,
-                                                   int h, bool upd, const float (&acc)[2][(P + 1) * (P + 1)],
-                                                   size_t k) {
+__device__ __forceinline__ void indicator_epilogue(const MixArgs& a, float* sd, int slot, int h, bool upd,
+                                                   const float (&acc)[2][(P + 1) * (P + 1)], size_t k) {
     constexpr int NQ = P + 1, NM = NQ * NQ, VP = vpitch(NM);
+    static_assert(kFeatureWord > 0 && kFeatureWord + kFeatureWords <= 3 * NM, "the means stay in place");
+    static_assert(TX == 16, "a warp's 16 cells are one row of the tile: consecutive slots");
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, row = pair_cell(lane);
-    float f[20];
-#pragma unroll
-    for (int i = 0; i < 20; ++i) f[i] = 0.0f;
-    float dev = 0.0f;  // largest |feature| of this half: the deviation from a constant state
+    // the cell's and the neighbours' input means, and the largest |feature| of
+    // this half (the deviation from a constant state).  Multiplying by `is`
+    // keeps order, so it is formed from the largest unscaled value; the features
+    // themselves are formed only in a warp that runs the network (about 1 in 28
+    // at the four-quadrant case)
+    float is = 0.0f, x0 = 0.0f, dL = 0.0f, dR = 0.0f, dU = 0.0f, dD = 0.0f, dev = 0.0f;
     if (upd) {
         const int var = h ? 3 : 0;
         const float m0 = sd[slot * VP + var * NM];
         const float mL = sd[(slot - 1) * VP + var * NM], mR = sd[(slot + 1) * VP + var * NM];
         const float mU = sd[(slot - (TX + 2)) * VP + var * NM], mD = sd[(slot + (TX + 2)) * VP + var * NM];
-        const float sc = fmaxf(fmaxf(fmaxf(fabsf(m0), fabsf(mL)), fmaxf(fabsf(mR), fabsf(mU))), fabsf(mD)) + 1e-12f;
-        const float is = 1.0f / sc;
+        is = 1.0f / (fmaxf(fmaxf(fmaxf(fabsf(m0), fabsf(mL)), fmaxf(fabsf(mR), fabsf(mU))), fabsf(mD)) + 1e-12f);
+        x0 = __fsub_rn((h ? acc[1][0] : acc[0][0]) * is, 1.0f);
+        dL = mL - m0;
+        dR = mR - m0;
+        dU = mU - m0;
+        dD = mD - m0;
+        float d0 = 0.0f, d1 = 0.0f;
+#pragma unroll
+        for (int m = 1; m < NM; ++m) {
+            d0 = fmaxf(d0, fabsf(acc[0][m]));
+            d1 = fmaxf(d1, fabsf(acc[1][m]));
+        }
+        // a NaN feature counts as 0 here, as it would in a maximum over the features
+        dev = fmaxf(0.0f, fmaxf(fmaxf(fmaxf(fabsf(dL), fabsf(dR)), fmaxf(fabsf(dU), fabsf(dD))), h ? d1 : d0) * is);
+        dev = fmaxf(dev, fabsf(x0));
+    }
+    dev = fmaxf(dev, __shfl_xor_sync(FULL, dev, kPairLane));
+    const bool cand = upd && !(dev <= a.screen);
+    float z = -INFINITY;
+    const auto features = [&](float (&f)[20]) {
+#pragma unroll
+        for (int i = 0; i < 20; ++i) f[i] = 0.0f;
+        if (!upd) return;
 #pragma unroll
         for (int px = 0; px < NQ; ++px)
 #pragma unroll
             for (int py = 0; py < NQ; ++py) f[px * 4 + py] = (h ? acc[1][px * NQ + py] : acc[0][px * NQ + py]) * is;
-        f[0] = __fsub_rn(f[0], 1.0f);
-        f[16] = (mL - m0) * is;
-        f[17] = (mR - m0) * is;
-        f[18] = (mU - m0) * is;
-        f[19] = (mD - m0) * is;
-#pragma unroll
-        for (int i = 0; i < 20; ++i) dev = fmaxf(dev, fabsf(f[i]));
-    }
-    dev = fmaxf(dev, __shfl_xor_sync(FULL, dev, kPairLane));
-    const bool cand = upd && !(dev <= a.screen);
-    __syncthreads();  // every face integral is taken: the flux region may hold the feature tiles
-    const bool warp_runs = __any_sync(FULL, cand);
-    float z = -INFINITY;
-    if (warp_runs) {
-        uint16_t* tile = ftiles + (threadIdx.x >> 5) * 16 * MLP_TILE_KP;
-        uint32_t* trow = reinterpret_cast<uint32_t*>(tile + row * MLP_TILE_KP);
+        f[0] = x0;
+        f[16] = dL * is;
+        f[17] = dR * is;
+        f[18] = dU * is;
+        f[19] = dD * is;
+    };
+    if (__any_sync(FULL, cand)) {
+        float f[20];
+        features(f);
+        __syncwarp();  // both halves of every cell are past their reads of its slot
+        uint32_t* trow = reinterpret_cast<uint32_t*>(sd + slot * VP + kFeatureWord);
         // row layout (words of BF16 pairs): rho modes 0..7, E modes 8..15, rho
         // differences 16..17, E differences 18..19, zero padding 20..23
 #pragma unroll
@@ -872,13 +890,15 @@ __device__ __forceinline__ void indicator_epilogue(const MixArgs& a, const float
         trow[21 + 2 * h] = 0u;
         __syncwarp();
         float lo, hi;
-        mlp_logits16(a.mlp, tile, lane, lo, hi);
+        mlp_logits16<VP>(a.mlp, trow - row * VP, lane, lo, hi);
         const int src = 4 * (row & 7);
         const float zl = __shfl_sync(FULL, lo, src), zh = __shfl_sync(FULL, hi, src);
         if (cand) z = row < 8 ? zl : zh;
     }
     if (a.dbg && upd) {
         float* o = a.dbg + k * 41;
+        float f[20];
+        features(f);
 #pragma unroll
         for (int i = 0; i < 16; ++i) o[16 * h + i] = f[i];
 #pragma unroll
@@ -1158,7 +1178,9 @@ __device__ __forceinline__ double stage_tile_pair(const MixArgs& a, int j0, int 
     float theta = 1.0f;
     bool rho_clamp = false, e_fix = false;
     const bool in_range = gi >= 3 && gi < ny - 3 && gj >= 3 && gj < nx - 3;
-    const bool lim = a.limiter == ZK_LIMITER_REFERENCE && in_range;
+    // the indicator gates the TVB pass, never this limiter: its kernels carry
+    // none of the code below (registers: the P = 3 stage 3 spilled with it)
+    const bool lim = !MLP && a.limiter == ZK_LIMITER_REFERENCE && in_range;
     const unsigned lm = __ballot_sync(pm, lim);
     if (lim) {
         if (kd == KIND_UPDATED) {
@@ -1339,12 +1361,7 @@ __device__ __forceinline__ double stage_tile_pair(const MixArgs& a, int j0, int 
     };
     const double umax_cell = cell_phase();
     if constexpr (MLP) {
-        // feature tiles: the flux region, or after the stage's shared memory
-        constexpr size_t own = sizeof(float) * (VP * SD + NQ * 4 * fx_stride(MTY, TX) + NQ * 4 * fy_stride(MTY, TX)) + SD;
-        uint16_t* tiles = mlp_tiles_in_flux<P, MTY, TX>() ? reinterpret_cast<uint16_t*>(sfx)
-                                                     : reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(smem) +
-                                                                                   align16(own));
-        if (a.stage > 0) indicator_epilogue<P, TX>(a, sd, tiles, slot, h, inside && kd == KIND_UPDATED, acc, k);
+        if (a.stage > 0) indicator_epilogue<P, TX>(a, sd, slot, h, inside && kd == KIND_UPDATED, acc, k);
     }
     return umax_cell;
 }
@@ -1377,20 +1394,12 @@ constexpr int pair_thread_budget(int P) { return P == 1 ? 1024 : P == 3 ? 512 : 
 // ms (P = 3 with the reference limiter 5.237 vs 5.199).  32 x 2 (4 CTAs of
 // 128 threads, the same 16 warps per SM, halo 2.1x) ran 9% slower than 32 x 4.
 constexpr int kPairCols = 16, kPairRows = 8;
-// Shared memory of the single-problem pair kernel, with the indicator's
-// feature tiles when MLP.
-template <int P, bool MLP>
-constexpr size_t pair_smem_bytes() {
-    return MLP && !mlp_tiles_in_flux<P, kPairRows, kPairCols>()
-               ? align16(smem_bytes<P, kPairRows, kPairCols>()) + kMlpTileBytes
-               : smem_bytes<P, kPairRows, kPairCols>();
-}
-template <int P, bool MLP = false>
+template <int P>
 constexpr int pair_min_blocks() {
-    return batch_min_blocks(kPairCols * 2 * kPairRows, pair_thread_budget(P), pair_smem_bytes<P, MLP>());
+    return batch_min_blocks(kPairCols * 2 * kPairRows, pair_thread_budget(P), smem_bytes<P, kPairRows, kPairCols>());
 }
 template <int P, typename TIn, typename TOut, bool MLP>
-__global__ void __launch_bounds__(kPairCols * 2 * kPairRows, pair_min_blocks<P, MLP>())
+__global__ void __launch_bounds__(kPairCols * 2 * kPairRows, pair_min_blocks<P>())
     dg_stage_mixed_pair_kernel(MixArgs a) {
     extern __shared__ __align__(16) float smem[];
     chain_wait();
@@ -1502,7 +1511,7 @@ cudaError_t launch_one(const MixArgs& a, cudaStream_t s) {
     constexpr bool pair = TPC == 2;
     static_assert(pair || !MLP, "the fused indicator runs in the two-threads-per-cell kernel");
     constexpr int rows = pair ? kPairRows : 4, cols = pair ? kPairCols : MTX;
-    constexpr size_t sm = pair ? pair_smem_bytes<P, MLP>() : smem_bytes<P, rows>();
+    constexpr size_t sm = smem_bytes<P, rows, cols>();
     auto* kern = pair ? dg_stage_mixed_pair_kernel<P, TIn, TOut, MLP> : dg_stage_mixed_kernel<P, TIn, TOut>;
     static std::atomic<bool> attr_set[64];  // per device; any host thread may launch
     int dev = 0;
@@ -1616,6 +1625,7 @@ cudaError_t launch_dg_stage_mixed(int P, const void* cur, int in_fp64, const dou
     if (tpc != 1 && tpc != 2) tpc = dg_mixed_default_tpc(P);
     if (ind) {
         if (!dg_mixed_fuses_indicator(P)) return cudaErrorInvalidValue;
+        if (limiter == ZK_LIMITER_REFERENCE) return cudaErrorInvalidValue;  // not in the indicator's kernels
         a.mlp = static_cast<const MlpFrag*>(ind->mlp);
         a.list = ind->list;
         a.count = ind->count;
