@@ -5,14 +5,15 @@
 // is bit-identical to it.  It is also the plain FP64 GPU path the mixed
 // precision kernel is measured against.
 //
-// One CTA owns a 32 x 8 tile of cells.  It stages the tile plus a 3-cell halo
-// of the stage input in shared memory (ghost cells already replaced by their
-// fill source), reconstructs both face values of every cell and direction,
-// computes every x and y interface flux of the tile ONCE (the reference
-// computes each interface twice, from both neighbours; both evaluations see
-// the same six inputs in the same order and give the same bits), then forms dU
-// and the Shu-Osher combine for every cell of the tile, ghosts included,
-// exactly as the reference's whole-array Eigen expressions do.
+// One CTA owns a tile of 32 columns and 2, 8 or 16 rows (launch_stage chooses
+// by grid size).  It stages the tile plus a 3-cell halo of the stage input in
+// shared memory (ghost cells already replaced by their fill source),
+// reconstructs both face values of every cell and direction, computes every x
+// and y interface flux of the tile ONCE (the reference computes each interface
+// twice, from both neighbours; both evaluations see the same six inputs in the
+// same order and give the same bits), then forms dU and the Shu-Osher combine
+// for every cell of the tile, ghosts included, exactly as the reference's
+// whole-array Eigen expressions do.
 //
 // Bound: the FP64 pipe.  A cell's smoothness indicators in one direction serve
 // its left-biased value on one face and its right-biased value on the other
