@@ -1,25 +1,30 @@
 // FP64 division without branches, and several quotients over one denominator.
 //
-// The FP64 kernels divide up to 15 times per interface.  The compiler's divide
-// carries a range test and a call on its slow path each time, so consecutive
-// divisions cannot overlap, and every division starts from its own
-// reciprocal.  Here the caller vouches for the operands' ranges -- tested once
+// The FP64 kernels divide up to 15 times per interface, several times by the
+// same value.  Here the caller vouches for the operands' ranges -- tested once
 // for a whole tile of cells (plain_value) or for a state's four values (num_ok),
 // plus a test of the few denominators that differences form (in_range) -- and
 // takes plain `/` elsewhere; inside the range the quotients are straight-line
-// code.
+// code that overlaps, and those over one denominator share its reciprocal.
 //
 // Reference-arithmetic build: quotients are correctly rounded, hence bit for
-// bit those of `/`.  With y = RN(1/b) and q within one ulp of a/b,
-// RN(q + y RN(a - b q)) = RN(a/b) (P. Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
-// 1990, Theorem 8.1's correction step; the remainder is exact).  y starts from
-// the 20-bit hardware approximation y0: with e = 1 - b y0, the cubic step
-// y0 + y0 (e + e^2) leaves a relative error below 2^-53 + 2^-57, and one
-// Newton step from there rounds to RN(1/b) for every b but the all-ones
-// significand (in_range sends those to `/`).  RN(a y) is within 1.5 ulp of
-// a/b, so two correction steps follow: the first brings it within one ulp, the
-// second rounds.
+// bit those of `/`.  The method is P. Markstein's ("Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990):
+// Newton's iteration y <- y + y (1 - b y) for the reciprocal, then the
+// quotient corrected by its remainder, q <- q + y (a - b q), all with fused
+// multiply-adds.
+//   Reciprocal.  The hardware approximation is within 2^-19 of 1/b (measured
+// for every significand it distinguishes, tests/test_fp64_div_gpu.py).  Two
+// iterations leave half an ulp plus a relative 2^-75.  The third then adds an
+// exact residual: before rounding it is (1/b)(1 - d^2) with |d| < b 2^-54 +
+// 2^-75, b scaled to [1, 2).  It rounds as 1/b does unless a midpoint m of two
+// neighbouring values lies between, 0 < 1 - b m <= d^2.  1 - b m is a positive
+// multiple of 2^-106, so d^2 >= 2^-106 and b > 2 - 2^-20; with b = 2 - t 2^-52
+// that needs t^2 - 1 to be a multiple of 2^53 - t, which of t < 2^33 only t =
+// 1 is: the all-ones significand, which in_range sends to `/`.
+//   Quotient.  RN(a y) is within 2 ulp of a/b; the first correction brings it
+// within one, and from there RN(q + y (a - b q)) = RN(a/b) for y = RN(1/b)
+// (Markstein's theorem; the remainder is exact).
 //
 // FMA build (ZK_PREC_FP64_FMA): y within one ulp, quotients a y.
 #pragma once
@@ -64,10 +69,8 @@ template <bool EXACT>
 __device__ __forceinline__ double recip(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    double e = __fma_rn(-b, y, 1.0);
-    e = __fma_rn(e, e, e);
-    y = __fma_rn(y, e, y);
-    if constexpr (EXACT) y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+#pragma unroll
+    for (int k = 0; k < (EXACT ? 3 : 2); ++k) y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
     return y;
 }
 
