@@ -9,6 +9,10 @@
 // -> 19.  The first staged copy of a context page-locks 5 MB (3 to 5 ms), so
 // uploads, which lose less to the runtime, do not start it below 192 MB.
 //
+// The workers' copies run on a stream of the staging's own, behind an event of
+// the caller's: a stream handle may mean another stream in another thread
+// (cudaStreamPerThread), so only the calling thread uses the caller's.
+//
 // Small copies, copies of memory the caller has page-locked (the runtime
 // moves those directly) and copies on a stream being captured go to the
 // runtime unchanged, as do all copies when page-locked memory runs out.
@@ -26,6 +30,17 @@ constexpr int kWorkers = 5;
 constexpr size_t kChunk = size_t(512) << 10;      // bytes of one staging buffer
 constexpr size_t kStagedMin = size_t(4) << 20;    // smaller copies are not worth the threads
 constexpr size_t kAllocMin = size_t(24) << 20;    // nor smaller ones page-locking the buffers
+
+// Exempts this thread from the calls that another stream's capture forbids
+// (page-locking memory, waiting for an event): none of them concerns it.
+class CaptureExempt {
+public:
+    CaptureExempt() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~CaptureExempt() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+
+private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
 
 // Rows [r0, r1) of the copy through the worker's two buffers.
 template <bool TO_DEVICE>
@@ -73,8 +88,24 @@ cudaError_t move_rows(char* host, char* dev, size_t pitch, size_t width, size_t 
 }  // namespace
 
 void HostStage::release() {
+    const CaptureExempt exempt;
+    if (stream_) cudaStreamDestroy(stream_);
+    if (before_) cudaEventDestroy(before_);
     if (base_) cudaFreeHost(base_);
+    stream_ = nullptr;
+    before_ = nullptr;
     base_ = nullptr;
+}
+
+bool HostStage::allocate() {
+    const CaptureExempt exempt;
+    if (cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking) == cudaSuccess &&
+        cudaEventCreateWithFlags(&before_, cudaEventDisableTiming) == cudaSuccess &&
+        cudaHostAlloc(reinterpret_cast<void**>(&base_), 2 * kWorkers * kChunk, cudaHostAllocPortable) == cudaSuccess)
+        return true;
+    release();
+    cudaGetLastError();
+    return false;
 }
 
 bool HostStage::ready(bool to_device, const void* host, size_t bytes, size_t width, cudaStream_t s) {
@@ -87,12 +118,7 @@ bool HostStage::ready(bool to_device, const void* host, size_t bytes, size_t wid
         return false;
     }
     if (at.type != cudaMemoryTypeUnregistered || cs != cudaStreamCaptureStatusNone) return false;
-    if (!base_ && cudaHostAlloc(reinterpret_cast<void**>(&base_), 2 * kWorkers * kChunk, cudaHostAllocPortable) !=
-                      cudaSuccess) {
-        cudaGetLastError();
-        base_ = nullptr;
-    }
-    return base_ != nullptr;
+    return base_ || allocate();
 }
 
 template <bool TO_DEVICE>
@@ -104,13 +130,17 @@ cudaError_t HostStage::copy(char* host, char* dev, size_t pitch, size_t width, s
         return e != cudaSuccess ? e : cudaStreamSynchronize(s);
     }
     int device = 0;
-    cudaGetDevice(&device);
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaEventRecord(before_, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(stream_, before_);
+    if (e != cudaSuccess) return e;
     std::atomic<int> err{cudaSuccess};
     const auto work = [&](int w) {
+        const CaptureExempt exempt;
         cudaSetDevice(device);
-        const cudaError_t e = move_rows<TO_DEVICE>(host, dev, pitch, width, rows * w / kWorkers,
-                                                   rows * (w + 1) / kWorkers, base_ + 2 * w * kChunk, s);
-        if (e != cudaSuccess) err = e;
+        const cudaError_t r = move_rows<TO_DEVICE>(host, dev, pitch, width, rows * w / kWorkers,
+                                                   rows * (w + 1) / kWorkers, base_ + 2 * w * kChunk, stream_);
+        if (r != cudaSuccess) err = r;
     };
     std::thread threads[kWorkers];
     int started = 1;
@@ -121,7 +151,8 @@ cudaError_t HostStage::copy(char* host, char* dev, size_t pitch, size_t width, s
     work(0);
     for (int w = started; w < kWorkers; ++w) work(w);
     for (int w = 1; w < started; ++w) threads[w].join();
-    const cudaError_t e = cudaStreamSynchronize(s);
+    const CaptureExempt exempt;
+    e = cudaStreamSynchronize(stream_);  // uploads: every worker's last chunks
     return err != cudaSuccess ? static_cast<cudaError_t>(err.load()) : e;
 }
 

@@ -6,9 +6,9 @@
 
 namespace zk {
 
-// One context's (or batch's) staging buffers, page-locked, allocated at its
-// first large copy and freed with it.  Used by one host thread at a time, as
-// its owner is.
+// One context's (or batch's) staging buffers, page-locked, and the stream their
+// copies run on, made at its first large copy and freed with it.  Used by one
+// host thread at a time, as its owner is.
 class HostStage {
 public:
     HostStage() = default;
@@ -26,7 +26,10 @@ private:
     template <bool TO_DEVICE>
     cudaError_t copy(char* host, char* dev, size_t pitch, size_t width, size_t rows, cudaStream_t s);
     bool ready(bool to_device, const void* host, size_t bytes, size_t width, cudaStream_t s);
+    bool allocate();
     char* base_ = nullptr;
+    cudaStream_t stream_ = nullptr;
+    cudaEvent_t before_ = nullptr;  // the work on the caller's stream
 };
 
 }  // namespace zk
