@@ -2,16 +2,26 @@
 //
 // A step is a chain of dependent kernels of a few to a few hundred
 // microseconds.  Launched plainly, each starts only when its predecessor has
-// drained and been retired; launched chained, its CTAs take their places while
-// the predecessor's last CTAs still run, and wait there (chain_wait) until all
-// of its memory is visible.  Every kernel of a chain calls chain_wait in every
-// thread before it reads or writes anything another kernel writes or reads, so
-// completion stays transitive along the chain.  A predecessor that is not a
-// kernel, or that never signals, orders a chained launch like a plain one.
-// Plain against chained, a pass of perf/cases.py: weno_fp64_64 47 -> 42 us,
-// weno_mixed_173x301 55 -> 50, dg1_mixed_jet_512x1024 1,830 -> 1,765,
-// weno_mixed_2048 697 -> 681, dg2_mixed_wave_1030 7,640 -> 7,445,
-// dg3_mixed_2048 unchanged.
+// drained, been retired and its memory flushed; launched chained, its launch
+// overlaps that end, and its CTAs wait (chain_wait) until all of the
+// predecessor's memory is visible.  Every kernel of a chain calls chain_wait in
+// every thread before it reads or writes anything another kernel writes or
+// reads, so completion stays transitive along the chain.  A predecessor that is
+// not a kernel orders a chained launch like a plain one.
+//
+// No kernel triggers its dependents before it ends (griddepcontrol.
+// launch_dependents): a dependent's CTAs would then be placed around CTAs that
+// still run, some SMs taking several and others none, and they stay there.
+// Microseconds per step (graph replay, four-quadrant case), plainly launched /
+// triggering at kernel start / as here:
+//   WENO FP64 64^2                    16.8 /  18.9 /  15.8
+//   WENO mixed 512^2                  55.6 /  49.5 /  50.2
+//   DG P=1 mixed 128^2                17.6 /  24.7 /  16.2
+//   DG P=2 mixed 128^2                26.0 /  38.2 /  24.8
+//   DG P=3 FP64 96^2                  59.9 /  88.1 /  57.0
+//   DG P=3 mixed, TVB, 128^2          47.5 /  66.4 /  45.4
+//   DG P=2 mixed, TVB, 1024^2        714   / 703   / 701
+//   DG P=3 mixed, indicator, 2048^2 5125   /5143   /5119
 #pragma once
 
 #include <cuda_runtime.h>
@@ -19,7 +29,6 @@
 namespace zk {
 
 __device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
