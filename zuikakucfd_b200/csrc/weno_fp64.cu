@@ -131,21 +131,12 @@ __device__ __forceinline__ double muscl_slope(double a, double b) {
         return s1 * s2 <= 0.0 ? 0.0 : (fabs(s1) > fabs(s2) ? s1 : s2);
     }
 }
+// Both values of the face between u[1] and u[2] of four cells `st` apart.
 template <int LIM>
-__device__ __forceinline__ void muscl_cell(double B, double C, double D, double& left, double& right) {
-    const double dm = C - B, dp = D - C;
-    left = C + 0.5 * muscl_slope<LIM>(dm, dp);   // UL of face i+1/2: slopes dL, dC
-    right = C - 0.5 * muscl_slope<LIM>(dm, dp);  // UR of face i-1/2: slopes dC, dR
-}
-
-// The cell's values on its face i+1/2 (left) and i-1/2 (right): WENO5 (RECON 0,
-// the reference's scheme) or MUSCL with limiter RECON - 1, whose face values
-// depend on the cells i-1, i, i+1 alone.
-template <int RECON, bool PLAIN>
-__device__ __forceinline__ void cell_values(double A, double B, double C, double D, double E, double& left,
-                                            double& right) {
-    if constexpr (RECON == 0) weno5_cell<PLAIN>(A, B, C, D, E, left, right);
-    else muscl_cell<RECON - 1>(B, C, D, left, right);
+__device__ __forceinline__ void muscl_face(const double* u, int st, double& left, double& right) {
+    const double dL = u[st] - u[0], dC = u[2 * st] - u[st], dR = u[3 * st] - u[2 * st];
+    left = u[st] + 0.5 * muscl_slope<LIM>(dL, dC);
+    right = u[2 * st] - 0.5 * muscl_slope<LIM>(dC, dR);
 }
 
 // hllcFlux (WENO variant), src_WENO/fluid.cpp:268-317, with plain divisions:
@@ -277,13 +268,11 @@ struct Smem {
     int8_t sK[TY + 6][HX];
 };
 
-// The interface fluxes of a staged tile, each computed once, left in S.xl and
-// S.yl.  First both face values of every cell beside a face, one variable of a
-// row of cells per warp task: TY x rows (columns 0 .. 31), the columns -1 and
-// 32 of all x rows, TY + 2 y rows (rows -1 .. TY); then the fluxes, a row of
-// faces per warp task.
-template <int TY, int NW, int RECON, bool PLAIN>
-__device__ __forceinline__ void tile_fluxes(Smem<TY>& S, double gamma, bool edge) {
+// Both values of every face of a staged tile (WENO5), into S: one variable of
+// a row of cells per warp task, TY x rows (columns 0 .. 31), the columns -1 and
+// 32 of all x rows, TY + 2 y rows (rows -1 .. TY).
+template <int TY, int NW, bool PLAIN>
+__device__ __forceinline__ void weno5_faces(Smem<TY>& S, bool edge) {
     auto& sU = S.sU;
     auto& sK = S.sK;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -302,7 +291,7 @@ __device__ __forceinline__ void tile_fluxes(Smem<TY>& S, double gamma, bool edge
                 if (k[-1] != KIND_UPDATED && k[0] != KIND_UPDATED && k[1] != KIND_UPDATED) continue;
             }
             const double* u = &sU[q][r + 3][c + 3];
-            cell_values<RECON, PLAIN>(u[-2], u[-1], u[0], u[1], u[2], left, right);
+            weno5_cell<PLAIN>(u[-2], u[-1], u[0], u[1], u[2], left, right);
             if (c < TX) S.xl[q][r][c + 1] = left;
             if (c >= 0) S.xr[q][r][c] = right;
         } else {
@@ -312,12 +301,25 @@ __device__ __forceinline__ void tile_fluxes(Smem<TY>& S, double gamma, bool edge
                 if (k[-HX] != KIND_UPDATED && k[0] != KIND_UPDATED && k[HX] != KIND_UPDATED) continue;
             }
             const double* u = &sU[q][r + 3][c + 3];
-            cell_values<RECON, PLAIN>(u[-2 * HX], u[-HX], u[0], u[HX], u[2 * HX], left, right);
+            weno5_cell<PLAIN>(u[-2 * HX], u[-HX], u[0], u[HX], u[2 * HX], left, right);
             if (r < TY) S.yl[q][r + 1][c] = left;
             if (r >= 0) S.yr[q][r][c] = right;
         }
     }
     __syncthreads();
+}
+
+// The interface fluxes of a staged tile, each computed once, left in S.xl and
+// S.yl, a row of faces per warp task.  RECON 0: WENO5, the reference's scheme,
+// from its own pass over the cells; else MUSCL with limiter RECON - 1, whose
+// slopes are too few operations to pay for that pass and its barrier (a step
+// with minmod, by cells / by faces: 192^2 30.1 / 18.9 us, 1024^2 271 / 233).
+template <int TY, int NW, int RECON, bool PLAIN>
+__device__ __forceinline__ void tile_fluxes(Smem<TY>& S, double gamma, bool edge) {
+    auto& sU = S.sU;
+    auto& sK = S.sK;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (RECON == 0) weno5_faces<TY, NW, PLAIN>(S, edge);
     for (int task = warp; task < 2 * TY + 2; task += NW) {
         if (task <= TY) {
             // x face on the left of tile cell (r, c)
@@ -325,9 +327,16 @@ __device__ __forceinline__ void tile_fluxes(Smem<TY>& S, double gamma, bool edge
             if (task < TY) { r = task; c = lane; }
             else { if (lane >= TY) continue; r = lane; c = TX; }
             if (edge && sK[r + 3][c + 2] != KIND_UPDATED && sK[r + 3][c + 3] != KIND_UPDATED) continue;
-            const double L[4] = {S.xl[0][r][c], S.xl[1][r][c], S.xl[2][r][c], S.xl[3][r][c]};
-            const double R[4] = {S.xr[0][r][c], S.xr[1][r][c], S.xr[2][r][c], S.xr[3][r][c]};
-            double F[4];
+            double L[4], R[4], F[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if constexpr (RECON == 0) {
+                    L[q] = S.xl[q][r][c];
+                    R[q] = S.xr[q][r][c];
+                } else {
+                    muscl_face<RECON - 1>(&sU[q][r + 3][c + 1], 1, L[q], R[q]);
+                }
+            }
             if constexpr (PLAIN) hllc_plain(L, R, gamma, F);
             else hllc_any(L, R, gamma, F);
 #pragma unroll
@@ -336,15 +345,21 @@ __device__ __forceinline__ void tile_fluxes(Smem<TY>& S, double gamma, bool edge
             // y face above tile cell (r, c); normal momentum swapped in
             const int r = task - TY - 1, c = lane;
             if (edge && sK[r + 2][c + 3] != KIND_UPDATED && sK[r + 3][c + 3] != KIND_UPDATED) continue;
-            const double L[4] = {S.yl[0][r][c], S.yl[2][r][c], S.yl[1][r][c], S.yl[3][r][c]};
-            const double R[4] = {S.yr[0][r][c], S.yr[2][r][c], S.yr[1][r][c], S.yr[3][r][c]};
-            double F[4];
+            double L[4], R[4], F[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int v = q == 1 ? 2 : q == 2 ? 1 : q;
+                if constexpr (RECON == 0) {
+                    L[q] = S.yl[v][r][c];
+                    R[q] = S.yr[v][r][c];
+                } else {
+                    muscl_face<RECON - 1>(&sU[v][r + 1][c + 3], HX, L[q], R[q]);
+                }
+            }
             if constexpr (PLAIN) hllc_plain(L, R, gamma, F);
             else hllc_any(L, R, gamma, F);
-            S.yl[0][r][c] = F[0];
-            S.yl[1][r][c] = F[1];
-            S.yl[2][r][c] = F[2];
-            S.yl[3][r][c] = F[3];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) S.yl[q][r][c] = F[q];
         }
     }
 }
