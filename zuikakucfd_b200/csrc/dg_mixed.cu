@@ -1378,10 +1378,11 @@ constexpr size_t smem_bytes() {
            SXT * SY;
 }
 
-// resident CTAs per SM: 8 for P=1 (+5% over 3), 3 for P=2 (4 and 5 were
-// slower) and P=3 (bounded by shared memory)
+// resident CTAs per SM: 8 for P=1 (+5% over 3), 4 for P=2 (a step at 256^2,
+// 512 tiles: 3 CTAs 71.4 us, 4 CTAs 48.4; 2048^2: 2,985 and 2,884), 3 for P=3
+// (bounded by shared memory)
 template <int P, typename TIn, typename TOut>
-__global__ void __launch_bounds__(MTX * 4, P == 1 ? 8 : 3) dg_stage_mixed_kernel(MixArgs a) {
+__global__ void __launch_bounds__(MTX * 4, P == 1 ? 8 : P == 2 ? 4 : 3) dg_stage_mixed_kernel(MixArgs a) {
     extern __shared__ __align__(16) float smem[];
     chain_wait();
     stage_tile<P, TIn, TOut, 4>(a, blockIdx.x * MTX, blockIdx.y * 4, smem);
