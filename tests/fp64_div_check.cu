@@ -8,12 +8,12 @@ __global__ void check_kernel(int n, const double* a, const double* b, double* ou
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double seed;
         asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(seed) : "d"(b[i]));
-        const double y = zk::recip<true>(b[i]);
+        const double y = zk::recip(b[i]);
         const size_t N = n;
         out[i] = seed;
         out[N + i] = y;
-        out[2 * N + i] = zk::quot<true>(a[i], b[i], y);
-        out[3 * N + i] = zk::divide<true>(a[i], b[i]);
+        out[2 * N + i] = zk::quot(a[i], b[i], y);
+        out[3 * N + i] = zk::divide(a[i], b[i]);
         out[4 * N + i] = 1.0 / b[i];
         out[5 * N + i] = a[i] / b[i];
         out[6 * N + i] = __fma_rn(-b[i], seed, 1.0);

@@ -159,13 +159,12 @@ int dg_upload_tables(int P, const DGTab& T) {
 namespace {
 
 // Whether quotients of the momenta (and, whole, the energy) of state U by its
-// floored density may take the shared reciprocal (fp64_div.cuh); the contracted
-// build needs no more than a normal density.
+// floored density may take the shared reciprocal (fp64_div.cuh).
 __device__ __forceinline__ bool momenta_plain(double rho, const double U[4]) {
-    return in_range(rho) && rho < 0x1p100 && (kFma || (num_ok(U[1]) && num_ok(U[2])));
+    return in_range(rho) && rho < 0x1p100 && num_ok(U[1]) && num_ok(U[2]);
 }
 __device__ __forceinline__ bool state_plain(double rho, const double U[4]) {
-    return momenta_plain(rho, U) && (kFma || num_ok(U[3]));
+    return momenta_plain(rho, U) && num_ok(U[3]);
 }
 
 // eulerFluxX / eulerFluxY, src_DG/fluid.cpp:123-143 (floors 1e-3)
@@ -173,9 +172,9 @@ __device__ __forceinline__ void euler_flux(const double U[4], double gam, double
     const double eps = 1e-3;
     double rho = ref_max(U[0], eps), u, v;
     if (momenta_plain(rho, U)) {
-        const double y = recip<!kFma>(rho);
-        u = quot<!kFma>(U[1], rho, y);
-        v = quot<!kFma>(U[2], rho, y);
+        const double y = recip(rho);
+        u = quot(U[1], rho, y);
+        v = quot(U[2], rho, y);
     } else {
         u = U[1] / rho;
         v = U[2] / rho;
@@ -236,7 +235,6 @@ __device__ __noinline__ void hllc_dg_any(const double* L, const double* R, doubl
 // roots are over half of an interface's FP64 work (face pass with plain
 // division: P=3 1024^2 419 us, now 370; contracted build 768^2 269, now 196).
 __device__ __forceinline__ void hllc_dg(const double (&L)[4], const double (&R)[4], double gamma, double (&F)[4]) {
-    constexpr bool X = !kFma;
     const double eps = 1e-5;
     const double rhoL = ref_max(L[0], eps), rhoR = ref_max(R[0], eps);
     const double sqL = sqrt(rhoL), sqR = sqrt(rhoR);
@@ -244,16 +242,16 @@ __device__ __forceinline__ void hllc_dg(const double (&L)[4], const double (&R)[
     if (den < eps) den = eps;
     bool ok = state_plain(rhoL, L) && state_plain(rhoR, R) && in_range(den);
     if (ok) {
-        const double yL = recip<X>(rhoL), yR = recip<X>(rhoR), yd = recip<X>(den);
-        const double uL = quot<X>(L[1], rhoL, yL), vL = quot<X>(L[2], rhoL, yL), EL = quot<X>(L[3], rhoL, yL);
+        const double yL = recip(rhoL), yR = recip(rhoR), yd = recip(den);
+        const double uL = quot(L[1], rhoL, yL), vL = quot(L[2], rhoL, yL), EL = quot(L[3], rhoL, yL);
         const double pL = ref_max((gamma - 1.0) * (L[3] - 0.5 * rhoL * (uL * uL + vL * vL)), eps);
-        const double aL = sqrt(ref_max(quot<X>(gamma * pL, rhoL, yL), eps));
-        const double uR = quot<X>(R[1], rhoR, yR), vR = quot<X>(R[2], rhoR, yR), ER = quot<X>(R[3], rhoR, yR);
+        const double aL = sqrt(ref_max(quot(gamma * pL, rhoL, yL), eps));
+        const double uR = quot(R[1], rhoR, yR), vR = quot(R[2], rhoR, yR), ER = quot(R[3], rhoR, yR);
         const double pR = ref_max((gamma - 1.0) * (R[3] - 0.5 * rhoR * (uR * uR + vR * vR)), eps);
-        const double aR = sqrt(ref_max(quot<X>(gamma * pR, rhoR, yR), eps));
-        const double u_roe = quot<X>(sqL * uL + sqR * uR, den, yd);
+        const double aR = sqrt(ref_max(quot(gamma * pR, rhoR, yR), eps));
+        const double u_roe = quot(sqL * uL + sqR * uR, den, yd);
         const double h_roe =
-            quot<X>(sqL * (EL + quot<X>(pL, rhoL, yL)) + sqR * (ER + quot<X>(pR, rhoR, yR)), den, yd);
+            quot(sqL * (EL + quot(pL, rhoL, yL)) + sqR * (ER + quot(pR, rhoR, yR)), den, yd);
         const double c_roe = sqrt(ref_max((gamma - 1.0) * (h_roe - 0.5 * u_roe * u_roe), eps));
         const double SL = ref_min(uL - aL, u_roe - c_roe);
         const double SR = ref_max(uR + aR, u_roe + c_roe);
@@ -265,7 +263,7 @@ __device__ __forceinline__ void hllc_dg(const double (&L)[4], const double (&R)[
             const double num = pR - pL + rhoL * uL * (SL - uL) - rhoR * uR * (SR - uR);
             double den2 = rhoL * (SL - uL) - rhoR * (SR - uR);
             if (fabs(den2) < eps) den2 = (den2 >= 0 ? eps : -eps);
-            const double Ss = divide<X>(num, den2);
+            const double Ss = divide(num, den2);
             const bool left = (Ss >= 0.0);
             const double rho = left ? rhoL : rhoR, u = left ? uL : uR, v = left ? vL : vR;
             const double E = left ? EL : ER, p = left ? pL : pR, S = left ? SL : SR;
@@ -275,8 +273,8 @@ __device__ __forceinline__ void hllc_dg(const double (&L)[4], const double (&R)[
             if (fabs(denom) < eps) denom = (denom >= 0 ? eps : -eps);
             const double r = rho * (S - u);
             ok = in_range(den2) && in_range(denom) && in_range(r);
-            const double c = divide<X>(r, denom);
-            const double term = (Ss - u) * (Ss + divide<X>(p, r));  // finite: every factor is in range
+            const double c = divide(r, denom);
+            const double term = (Ss - u) * (Ss + divide(p, r));  // finite: every factor is in range
             F[0] = rho * u + S * (c - U0);
             F[1] = rho * u * u + p + S * (c * Ss - U1);
             F[2] = rho * u * v + S * (c * v - U2);

@@ -7,12 +7,13 @@
 // takes plain `/` elsewhere; inside the range the quotients are straight-line
 // code that overlaps, and those over one denominator share its reciprocal.
 //
-// Reference-arithmetic build: quotients are correctly rounded, hence bit for
-// bit those of `/`.  The method is P. Markstein's ("Computation of elementary
-// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990):
-// Newton's iteration y <- y + y (1 - b y) for the reciprocal, then the
-// quotient corrected by its remainder, q <- q + y (a - b q), all with fused
-// multiply-adds.
+// Quotients are correctly rounded, hence bit for bit those of `/`, in the
+// reference-arithmetic build and in the contracted one (ZK_PREC_FP64_FMA fuses
+// multiply-adds and changes nothing else).  The method is P. Markstein's
+// ("Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990): Newton's iteration
+// y <- y + y (1 - b y) for the reciprocal, then the quotient corrected by its
+// remainder, q <- q + y (a - b q), all with fused multiply-adds.
 //   Reciprocal.  The hardware approximation is within 2^-19 of 1/b (measured
 // for every significand it distinguishes, tests/test_fp64_div_gpu.py).  Two
 // iterations leave half an ulp plus a relative 2^-75.  The third then adds an
@@ -25,8 +26,6 @@
 //   Quotient.  RN(a y) is within 2 ulp of a/b; the first correction brings it
 // within one, and from there RN(q + y (a - b q)) = RN(a/b) for y = RN(1/b)
 // (Markstein's theorem; the remainder is exact).
-//
-// FMA build (ZK_PREC_FP64_FMA): y within one ulp, quotients a y.
 #pragma once
 
 #include <cstdint>
@@ -64,30 +63,23 @@ __device__ __forceinline__ bool plain_value(double a) {
     return h - 0x33700000u < 0x10400000u || (h | __double2loint(a)) == 0;
 }
 
-// 1/b for in_range(b): RN (see above), or within one ulp when !EXACT.
-template <bool EXACT>
+// RN(1/b) for in_range(b).
 __device__ __forceinline__ double recip(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
 #pragma unroll
-    for (int k = 0; k < (EXACT ? 3 : 2); ++k) y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    for (int k = 0; k < 3; ++k) y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
     return y;
 }
 
-// a/b, given y = recip<EXACT>(b).
-template <bool EXACT>
+// RN(a/b), given y = recip(b).
 __device__ __forceinline__ double quot(double a, double b, double y) {
     double q = __dmul_rn(a, y);
-    if constexpr (EXACT) {
-        q = __fma_rn(__fma_rn(-b, q, a), y, q);
-        q = __fma_rn(__fma_rn(-b, q, a), y, q);
-    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) q = __fma_rn(__fma_rn(-b, q, a), y, q);
     return q;
 }
 
-template <bool EXACT>
-__device__ __forceinline__ double divide(double a, double b) {
-    return quot<EXACT>(a, b, recip<EXACT>(b));
-}
+__device__ __forceinline__ double divide(double a, double b) { return quot(a, b, recip(b)); }
 
 }  // namespace zk

@@ -45,12 +45,6 @@ namespace ZK_FP64_NS {
 using namespace zk;
 namespace {
 
-#ifdef ZK_FP64_FMA
-constexpr bool kExact = false;
-#else
-constexpr bool kExact = true;  // quotients correctly rounded
-#endif
-
 // A tile is 32 x TY cells; NW warps (TY + 1 by default) take the 2 TY + 2
 // face-row tasks (TY + 1 x-face rows, TY + 1 y-face rows) in turn.
 constexpr int TX = 32, HX = TX + 6;
@@ -72,16 +66,16 @@ __device__ __forceinline__ void weno5_weights(double t0, double t1, double t2, d
                                               double& ia, double& ie) {
     const double q0 = t0 * t0, q1 = t1 * t1, q2 = t2 * t2;
     if (PLAIN && !ones_low(q0, q1, q2)) {
-        const double y0 = recip<kExact>(q0), y1 = recip<kExact>(q1), y2 = recip<kExact>(q2);
-        a[0] = quot<kExact>(0.1, q0, y0);
-        a[1] = e[1] = quot<kExact>(0.6, q1, y1);
-        a[2] = quot<kExact>(0.3, q2, y2);
-        e[0] = quot<kExact>(0.1, q2, y2);
-        e[2] = quot<kExact>(0.3, q0, y0);
+        const double y0 = recip(q0), y1 = recip(q1), y2 = recip(q2);
+        a[0] = quot(0.1, q0, y0);
+        a[1] = e[1] = quot(0.6, q1, y1);
+        a[2] = quot(0.3, q2, y2);
+        e[0] = quot(0.1, q2, y2);
+        e[2] = quot(0.3, q0, y0);
         const double sa = a[0] + a[1] + a[2], se = e[0] + e[1] + e[2];
         if (!ones_low(sa, se)) {
-            ia = recip<kExact>(sa);
-            ie = recip<kExact>(se);
+            ia = recip(sa);
+            ie = recip(se);
             return;
         }
     }
@@ -189,23 +183,22 @@ __device__ __noinline__ void hllc_any(const double* L, const double* R, double g
 // quotient and remainder below is normal unless a difference underflows or
 // vanishes: den2, r and d are tested.
 __device__ __forceinline__ void hllc_plain(const double (&L)[4], const double (&R)[4], double gamma, double (&F)[4]) {
-    constexpr bool X = kExact;
     const double eps = 1e-12;
     const double rhoL = ref_max(L[0], eps), rhoR = ref_max(R[0], eps);
     const double sqL = sqrt(rhoL), sqR = sqrt(rhoR), den = sqL + sqR;
     bool ok = !ones_low(rhoL, rhoR, den);
     {
-        const double yL = recip<X>(rhoL), yR = recip<X>(rhoR);
-        const double uL = quot<X>(L[1], rhoL, yL), vL = quot<X>(L[2], rhoL, yL), EL = quot<X>(L[3], rhoL, yL);
+        const double yL = recip(rhoL), yR = recip(rhoR);
+        const double uL = quot(L[1], rhoL, yL), vL = quot(L[2], rhoL, yL), EL = quot(L[3], rhoL, yL);
         const double pL = ref_max((gamma - 1.0) * (L[3] - 0.5 * rhoL * (uL * uL + vL * vL)), eps);
-        const double aL = sqrt(quot<X>(gamma * pL, rhoL, yL));
-        const double uR = quot<X>(R[1], rhoR, yR), vR = quot<X>(R[2], rhoR, yR), ER = quot<X>(R[3], rhoR, yR);
+        const double aL = sqrt(quot(gamma * pL, rhoL, yL));
+        const double uR = quot(R[1], rhoR, yR), vR = quot(R[2], rhoR, yR), ER = quot(R[3], rhoR, yR);
         const double pR = ref_max((gamma - 1.0) * (R[3] - 0.5 * rhoR * (uR * uR + vR * vR)), eps);
-        const double aR = sqrt(quot<X>(gamma * pR, rhoR, yR));
-        const double yd = recip<X>(den);
-        const double u_roe = quot<X>(sqL * uL + sqR * uR, den, yd);
+        const double aR = sqrt(quot(gamma * pR, rhoR, yR));
+        const double yd = recip(den);
+        const double u_roe = quot(sqL * uL + sqR * uR, den, yd);
         const double h_roe =
-            quot<X>(sqL * (EL + quot<X>(pL, rhoL, yL)) + sqR * (ER + quot<X>(pR, rhoR, yR)), den, yd);
+            quot(sqL * (EL + quot(pL, rhoL, yL)) + sqR * (ER + quot(pR, rhoR, yR)), den, yd);
         const double c_roe = sqrt(ref_max((gamma - 1.0) * (h_roe - 0.5 * u_roe * u_roe), eps));
         const double SL = ref_min(uL - aL, u_roe - c_roe);
         const double SR = ref_max(uR + aR, u_roe + c_roe);
@@ -217,7 +210,7 @@ __device__ __forceinline__ void hllc_plain(const double (&L)[4], const double (&
             const double num = pR - pL + rhoL * uL * (SL - uL) - rhoR * uR * (SR - uR);
             double den2 = rhoL * (SL - uL) - rhoR * (SR - uR);
             if (fabs(den2) < 1e-12) den2 = (den2 >= 0 ? 1e-12 : -1e-12);
-            const double Ss = divide<X>(num, den2);
+            const double Ss = divide(num, den2);
             const bool left = (Ss >= 0.0);
             const double rho = left ? rhoL : rhoR, u = left ? uL : uR, v = left ? vL : vR;
             const double E = left ? EL : ER, p = left ? pL : pR, S = left ? SL : SR;
@@ -225,8 +218,8 @@ __device__ __forceinline__ void hllc_plain(const double (&L)[4], const double (&
                          U3 = left ? L[3] : R[3];
             const double r = rho * (S - u), d = S - Ss;
             ok = ok && in_range(den2) && in_range(r) && in_range(d);
-            const double c = divide<X>(r, d);
-            const double s3 = c * (E + (Ss - u) * (Ss + divide<X>(p, r)));
+            const double c = divide(r, d);
+            const double s3 = c * (E + (Ss - u) * (Ss + divide(p, r)));
             F[0] = rho * u + S * (c - U0);
             F[1] = rho * u * u + p + S * (c * Ss - U1);
             F[2] = rho * u * v + S * (c * v - U2);
