@@ -83,4 +83,17 @@ def test_quotients_are_those_of_plain_division(check, kind_a, kind_b, ea, eb):
     bits = {k: v.view(np.uint64)[ok] for k, v in got.items()}
     assert np.array_equal(bits["recip"], bits["one_over"])
     assert np.array_equal(bits["divide"], bits["plain"])
-    assert np.array_equal(bits["quot"], bits["plain"])
+    pos = (b > 0)[ok]
+    assert np.array_equal(bits["quot"][pos], bits["plain"][pos])
+
+
+def test_signed_zeros(check):
+    """quot keeps the sign of either zero over a positive denominator, divide
+    that of +0 over any."""
+    r = np.random.default_rng(1)
+    b = compose(significands("any", r), r.integers(-60, 220, N), r.integers(0, 2, N))
+    a = np.where(r.integers(0, 2, N) == 1, 0.0, -0.0)
+    ok = (b.view(np.uint64) & 0xffffffff) != 0xffffffff
+    for name, sel in (("quot", ok & (b > 0)), ("divide", ok & ~np.signbit(a))):
+        got = check(a[sel], b[sel])
+        assert np.array_equal(got[name].view(np.uint64), got["plain"].view(np.uint64)), name

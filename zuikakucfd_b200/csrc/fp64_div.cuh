@@ -39,8 +39,8 @@ __device__ __forceinline__ bool in_range(double x) {
     return (uint32_t)((__double2hiint(x) & 0x7fffffff) - 0x20b00000) < 0x3e800000u && __double2loint(x) != -1;
 }
 
-// a == +0 (the quotient of a -0 would lose its sign) or |a| in [2^-300, 2^100):
-// conserved values whose quotients by a density in [1e-5, 2^100), and the
+// a == +0 (face and point values are sums that start from +0, never -0) or |a|
+// in [2^-300, 2^100): conserved values whose quotients by a density in [1e-5, 2^100), and the
 // fluxes' second-level quotients of those, stay above 2^-800 and below 2^700.
 __device__ __forceinline__ bool num_ok(double a) {
     const int h = __double2hiint(a);
@@ -72,14 +72,23 @@ __device__ __forceinline__ double recip(double b) {
     return y;
 }
 
-// RN(a/b), given y = recip(b).
+// RN(a/b) for b > 0, given y = recip(b).  The remainder is formed as b q - a:
+// for a = -0 that is +0, subtracting it keeps the quotient -0, and so with +0.
 __device__ __forceinline__ double quot(double a, double b, double y) {
+    double q = __dmul_rn(a, y);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) q = __fma_rn(-__fma_rn(b, q, -a), y, q);
+    return q;
+}
+
+// RN(a/b) for b of either sign and a other than -0 (with this sign of the
+// remainder, +0 keeps its quotient's sign over a negative b).
+__device__ __forceinline__ double divide(double a, double b) {
+    const double y = recip(b);
     double q = __dmul_rn(a, y);
 #pragma unroll
     for (int k = 0; k < 2; ++k) q = __fma_rn(__fma_rn(-b, q, a), y, q);
     return q;
 }
-
-__device__ __forceinline__ double divide(double a, double b) { return quot(a, b, recip(b)); }
 
 }  // namespace zk
