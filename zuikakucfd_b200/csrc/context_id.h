@@ -1,8 +1,9 @@
 // Identity of the current CUDA context, for state cached per context: a device
 // reset (cudaDeviceReset anywhere in the process) drops what the runtime held
-// for the old one (symbol addresses, kernel attributes).
+// for the old one (symbol addresses and contents, kernel attributes).
 #pragma once
 
+#include <atomic>
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <mutex>
@@ -35,5 +36,30 @@ inline bool current_context_id(unsigned long long* id) {
     if (get_current(&ctx) != CUDA_SUCCESS || !ctx) return false;
     return get_id(ctx, id) == CUDA_SUCCESS;
 }
+
+// What has been set up in each device's current context, once per kind of
+// set-up (a static object).
+class PerContext {
+public:
+    // Runs `set` unless it has run in the current device's context; any host
+    // thread may call.  Without a context id (old driver) it runs every time.
+    template <typename Set>
+    cudaError_t once(Set set) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        unsigned long long id = 0;
+        const bool slot = dev >= 0 && dev < 64;
+        if (slot && current_context_id(&id) && done_[dev].load(std::memory_order_acquire) == id + 1) return cudaSuccess;
+        e = set();
+        // the runtime calls above made the context current if it was not
+        if (e == cudaSuccess && slot && current_context_id(&id))
+            done_[dev].store(id + 1, std::memory_order_release);
+        return e;
+    }
+
+private:
+    std::atomic<unsigned long long> done_[64] = {};  // context id + 1
+};
 
 }  // namespace zk

@@ -22,6 +22,7 @@
 
 #include "batch.cuh"
 #include "chain.cuh"
+#include "context_id.h"
 #include "dg_common.cuh"
 #include "fp64_div.cuh"
 #include "zk_internal.h"
@@ -144,16 +145,13 @@ void dg_make_sep(int P, DGSep* S) {
 }
 
 int dg_upload_tables(int P, const DGTab& T) {
-    // __constant__ memory is per device: upload once per (device, P)
+    // __constant__ memory is per CUDA context: upload once per (context, P)
     static std::mutex mu;
-    static uint64_t done[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ZK_ERR_CUDA;
+    static PerContext uploaded[DG_MAXNQ];
     std::lock_guard<std::mutex> lock(mu);
-    if (done[dev] & (1ull << P)) return ZK_OK;
-    if (cudaMemcpyToSymbol(c_dgtab, &T, sizeof(DGTab), sizeof(DGTab) * (P - 1)) != cudaSuccess) return ZK_ERR_CUDA;
-    done[dev] |= (1ull << P);
-    return ZK_OK;
+    const cudaError_t e = uploaded[P].once(
+        [&] { return cudaMemcpyToSymbol(c_dgtab, &T, sizeof(DGTab), sizeof(DGTab) * (P - 1)); });
+    return e == cudaSuccess ? ZK_OK : ZK_ERR_CUDA;
 }
 
 namespace {

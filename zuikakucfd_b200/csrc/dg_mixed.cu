@@ -13,7 +13,6 @@
 // changes.  This file is compiled with --use_fast_math (FP32 division, sqrt,
 // log10 and sin use the MUFU approximations); the combine and limiter
 // arithmetic is rounded explicitly, so both kernels give the same bits.
-#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -22,6 +21,7 @@
 
 #include "batch.cuh"
 #include "chain.cuh"
+#include "context_id.h"
 #include "dg_common.cuh"
 #include "mlp_infer.cuh"
 #include "zk_internal.h"
@@ -1475,15 +1475,12 @@ template <int P, int STAGE, int V>
 cudaError_t batch_one(const DgItem* items, const int* dir, int cap, int grid, cudaStream_t s, int* occ) {
     constexpr size_t sm = smem_bytes<P, dg_variant_rows(V)>();
     constexpr int nt = MTX * dg_variant_rows(V) * dg_variant_tpc(V);
-    static std::atomic<bool> attr_set[64];  // per device; any host thread may launch
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(dg_stage_mixed_batch_kernel<P, STAGE, V>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        attr_set[dev].store(true, std::memory_order_release);
-    }
+    static PerContext attributes;
+    const cudaError_t e = attributes.once([] {
+        return cudaFuncSetAttribute(dg_stage_mixed_batch_kernel<P, STAGE, V>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    });
+    if (e != cudaSuccess) return e;
     if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, dg_stage_mixed_batch_kernel<P, STAGE, V>, nt, sm);
     dg_stage_mixed_batch_kernel<P, STAGE, V><<<grid, nt, sm, s>>>(items, dir, cap);
     return cudaGetLastError();
@@ -1519,14 +1516,10 @@ cudaError_t launch_one(const MixArgs& a, cudaStream_t s) {
     constexpr int rows = pair ? kPairRows : 4, cols = pair ? kPairCols : MTX;
     constexpr size_t sm = smem_bytes<P, rows, cols>();
     auto* kern = pair ? dg_stage_mixed_pair_kernel<P, TIn, TOut, MLP> : dg_stage_mixed_kernel<P, TIn, TOut>;
-    static std::atomic<bool> attr_set[64];  // per device; any host thread may launch
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        attr_set[dev].store(true, std::memory_order_release);
-    }
+    static PerContext attributes;
+    const cudaError_t e =
+        attributes.once([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); });
+    if (e != cudaSuccess) return e;
     dim3 grid((a.g.nx + cols - 1) / cols, (a.g.ny + rows - 1) / rows);
     return launch_chained(kern, grid, cols * rows * TPC, sm, s, a);
 }
@@ -1548,39 +1541,39 @@ cudaError_t launch_p(const MixArgs& a, int in_fp64, int out_fp64, int tpc, cudaS
 
 }  // namespace
 
-// FP32 copy of P's basis tables in this file's constant bank (once per device, P).
+// FP32 copy of P's basis tables in this file's constant bank (once per CUDA
+// context and P).
 int dg_upload_tables_f32(int P) {
     static std::mutex mu;
-    static uint64_t done[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ZK_ERR_CUDA;
+    static PerContext uploaded[DG_MAXNQ];
     std::lock_guard<std::mutex> lock(mu);
-    if (done[dev] & (1ull << P)) return ZK_OK;
-    DGTab T;
-    dg_make_tables(P, &T);
-    DGTabF F;
-    std::memset(&F, 0, sizeof F);
-    const double* src = reinterpret_cast<const double*>(&T);
-    float* dst = reinterpret_cast<float*>(&F);
-    static_assert(sizeof(DGTab) / sizeof(double) == sizeof(DGTabF) / sizeof(float), "table layouts differ");
-    for (size_t i = 0; i < sizeof(DGTab) / sizeof(double); ++i) dst[i] = (float)src[i];
-    if (cudaMemcpyToSymbol(c_tabf, &F, sizeof F, sizeof F * (P - 1)) != cudaSuccess) return ZK_ERR_CUDA;
-    DGSep S;
-    dg_make_sep(P, &S);
-    DGSepF SF;
-    std::memset(&SF, 0, sizeof SF);
-    for (int n = 0; n < DG_MAXNQ; ++n) {
-        for (int q = 0; q < DG_MAXNQ; ++q) {
-            SF.L[n][q] = (float)S.L[n][q];
-            SF.D[n][q] = (float)S.D[n][q];
-            SF.WL[n][q] = (float)(S.W[q] * S.L[n][q]);
+    const cudaError_t e = uploaded[P].once([&] {
+        DGTab T;
+        dg_make_tables(P, &T);
+        DGTabF F;
+        std::memset(&F, 0, sizeof F);
+        const double* src = reinterpret_cast<const double*>(&T);
+        float* dst = reinterpret_cast<float*>(&F);
+        static_assert(sizeof(DGTab) / sizeof(double) == sizeof(DGTabF) / sizeof(float), "table layouts differ");
+        for (size_t i = 0; i < sizeof(DGTab) / sizeof(double); ++i) dst[i] = (float)src[i];
+        const cudaError_t r = cudaMemcpyToSymbol(c_tabf, &F, sizeof F, sizeof F * (P - 1));
+        if (r != cudaSuccess) return r;
+        DGSep S;
+        dg_make_sep(P, &S);
+        DGSepF SF;
+        std::memset(&SF, 0, sizeof SF);
+        for (int n = 0; n < DG_MAXNQ; ++n) {
+            for (int q = 0; q < DG_MAXNQ; ++q) {
+                SF.L[n][q] = (float)S.L[n][q];
+                SF.D[n][q] = (float)S.D[n][q];
+                SF.WL[n][q] = (float)(S.W[q] * S.L[n][q]);
+            }
+            SF.W[n] = (float)S.W[n];
+            for (int a = 0; a < 4; ++a) SF.Z[n][a] = (float)S.Z[n][a];
         }
-        SF.W[n] = (float)S.W[n];
-        for (int a = 0; a < 4; ++a) SF.Z[n][a] = (float)S.Z[n][a];
-    }
-    if (cudaMemcpyToSymbol(c_sepf, &SF, sizeof SF, sizeof SF * (P - 1)) != cudaSuccess) return ZK_ERR_CUDA;
-    done[dev] |= (1ull << P);
-    return ZK_OK;
+        return cudaMemcpyToSymbol(c_sepf, &SF, sizeof SF, sizeof SF * (P - 1));
+    });
+    return e == cudaSuccess ? ZK_OK : ZK_ERR_CUDA;
 }
 
 // One mixed-precision DG stage of a batch group (grid persistent CTAs).

@@ -23,8 +23,6 @@
 // instructions per interface become 780: 177 -> 156 us a stage at 1024^2 (FP64
 // pipe 64%; the staging, combine and barrier phases of three CTAs per SM leave
 // the rest).
-#include <atomic>
-
 #include "batch.cuh"
 #include "chain.cuh"
 #include "context_id.h"
@@ -509,28 +507,12 @@ template <auto kernel>
 cudaError_t set_smem(size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
-// Runs `set` (kernel attributes) unless it has run in the current device's
-// context; any host thread may launch.  `done`: context id per device.
-template <typename Set>
-cudaError_t once_per_context(std::atomic<unsigned long long> (&done)[64], Set set) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    unsigned long long id = 0;
-    const bool known = dev >= 0 && dev < 64 && current_context_id(&id);
-    if (known && done[dev].load(std::memory_order_acquire) == id + 1) return cudaSuccess;
-    e = set();
-    // the runtime calls above made the context current if it was not
-    if (e == cudaSuccess && dev >= 0 && dev < 64 && current_context_id(&id))
-        done[dev].store(id + 1, std::memory_order_release);
-    return e;
-}
 template <int V>
 constexpr size_t batch_smem() { return sizeof(Smem<weno_variant_rows(V)>); }
 template <int V>
 cudaError_t batch_ready() {
-    static std::atomic<unsigned long long> done[64];
-    return once_per_context(done, [] { return set_smem<weno_stage_fp64_batch_kernel<V>>(batch_smem<V>()); });
+    static PerContext attributes;
+    return attributes.once([] { return set_smem<weno_stage_fp64_batch_kernel<V>>(batch_smem<V>()); });
 }
 template <int V>
 cudaError_t launch_batch_v(const WenoItem* items, const int* dir, int cap, int stage, int grid, cudaStream_t s) {
@@ -572,8 +554,8 @@ cudaError_t launch_stage(const StageArgs& a, cudaStream_t s) {
     constexpr int kSms = 148;
     // every tile height at once: a later call with another grid may be inside a
     // stream capture, where no kernel should be loaded for the first time
-    static std::atomic<unsigned long long> done[64];
-    const cudaError_t e = once_per_context(done, [] {
+    static PerContext attributes;
+    const cudaError_t e = attributes.once([] {
         cudaError_t r = set_smem<weno_stage_fp64_kernel<RECON, 8, 9, 3>>(sizeof(Smem<8>));
         if constexpr (RECON == 0) {
             if (r == cudaSuccess) r = set_smem<weno_stage_fp64_kernel<0, 2, 14, 2>>(sizeof(Smem<2>));
