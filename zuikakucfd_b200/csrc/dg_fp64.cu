@@ -439,11 +439,13 @@ __device__ __forceinline__ void face_tile(const DGArgs& a, int j0, int i, FaceTi
     }
 }
 
-template <int P>
-__global__ void __launch_bounds__(FaceTile<P>::NTHREAD) dg_face_kernel(DGArgs a) {
+// Rows 3 .. ny-3 hold every face of an updated cell; TALL: from row `row0`, a
+// variant of its own since the addition alone made the pass 1 to 4% longer.
+template <int P, bool TALL>
+__global__ void __launch_bounds__(FaceTile<P>::NTHREAD) dg_face_kernel(DGArgs a, int row0) {
     __shared__ FaceTile<P> S;
     chain_wait();
-    face_tile<P>(a, blockIdx.x * 32, 3 + blockIdx.y, S);  // rows 3 .. ny-3 hold every face of an updated cell
+    face_tile<P>(a, blockIdx.x * 32, (TALL ? row0 : 3) + blockIdx.y, S);
 }
 
 // ---- cells ---------------------------------------------------------------------------
@@ -973,11 +975,11 @@ __device__ __forceinline__ double cell_tile(const DGArgs& a, int j0, int i, Cell
 // 6 over 5 CTAs +1.2%; P=3: 5 CTAs at 100 registers the same time).
 constexpr int cell_ctas(int P) { return P == 3 ? 4 : P == 2 ? 6 : 12; }
 
-template <int P>
-__global__ void __launch_bounds__(CellTile<P>::NTHREAD, cell_ctas(P)) dg_cell_kernel(DGArgs a) {
+template <int P, bool TALL>  // TALL: as dg_face_kernel
+__global__ void __launch_bounds__(CellTile<P>::NTHREAD, cell_ctas(P)) dg_cell_kernel(DGArgs a, int row0) {
     __shared__ CellTile<P> S;
     chain_wait();
-    cell_tile<P>(a, blockIdx.x * 32, blockIdx.y, S);
+    cell_tile<P>(a, blockIdx.x * 32, TALL ? row0 + blockIdx.y : blockIdx.y, S);
 }
 
 #ifndef ZK_FP64_FMA  // the batched runner has no FP64_FMA groups
@@ -1090,10 +1092,21 @@ __global__ void __launch_bounds__(CellTile<P>::NTHREAD) dg_limit_kernel(DGArgs a
 
 template <int P>
 cudaError_t launch_stage(const DGArgs& a, cudaStream_t s) {
-    const int segs = (a.g.nx + 31) / 32;
-    const cudaError_t e = launch_chained(dg_face_kernel<P>, dim3(segs, a.g.ny - 5), FaceTile<P>::NTHREAD, 0, s, a);
-    if (e != cudaSuccess) return e;
-    return launch_chained(dg_cell_kernel<P>, dim3(segs, a.g.ny), CellTile<P>::NTHREAD, 0, s, a);
+    constexpr int kRows = 65535;  // gridDim.y
+    const int segs = (a.g.nx + 31) / 32, ny = a.g.ny, faces = ny - 5;
+    cudaError_t e = cudaSuccess;
+    if (ny <= kRows) {
+        e = launch_chained(dg_face_kernel<P, false>, dim3(segs, faces), FaceTile<P>::NTHREAD, 0, s, a, 0);
+        if (e != cudaSuccess) return e;
+        return launch_chained(dg_cell_kernel<P, false>, dim3(segs, ny), CellTile<P>::NTHREAD, 0, s, a, 0);
+    }
+    for (int r = 0; r < faces && e == cudaSuccess; r += kRows)
+        e = launch_chained(dg_face_kernel<P, true>, dim3(segs, faces - r < kRows ? faces - r : kRows),
+                           FaceTile<P>::NTHREAD, 0, s, a, 3 + r);
+    for (int r = 0; r < ny && e == cudaSuccess; r += kRows)
+        e = launch_chained(dg_cell_kernel<P, true>, dim3(segs, ny - r < kRows ? ny - r : kRows),
+                           CellTile<P>::NTHREAD, 0, s, a, r);
+    return e;
 }
 
 template <int P>
