@@ -45,7 +45,9 @@ cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, unsigned thread
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+    if (e != cudaSuccess) cudaGetLastError();  // reported here, not again by the next launch that asks for it
+    return e;
 }
 
 }  // namespace zk
