@@ -54,6 +54,15 @@ void free_device(zk_ctx* c) {
     c->d_status = nullptr;
 }
 
+// What zk_create made (and h_max, made with the first mesh), and the context.
+void release_context(zk_ctx* c) {
+    if (c->ev0) cudaEventDestroy(c->ev0);
+    if (c->ev1) cudaEventDestroy(c->ev1);
+    if (c->own_stream) cudaStreamDestroy(c->own_stream);
+    if (c->h_max) cudaFreeHost(c->h_max);
+    delete c;
+}
+
 }  // namespace
 
 // Ghost source map on the host, pitched indices.  The reference fills ghosts
@@ -168,11 +177,8 @@ int zk_create(const zk_options* opt, zk_ctx** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
-    if (e == cudaSuccess)
-        e = cudaHostAlloc(reinterpret_cast<void**>(&c->h_max), sizeof *c->h_max,
-                          cudaHostAllocMapped | cudaHostAllocPortable);
     if (e != cudaSuccess) {
-        delete c;
+        release_context(c);
         return fail(ZK_ERR_CUDA, "context setup: %s", cudaGetErrorString(e));
     }
     c->stream = c->own_stream;
@@ -186,11 +192,7 @@ int zk_destroy(zk_ctx* c) {
     cudaStreamSynchronize(c->stream);
     free_device(c);
     zk_dg_release(c);
-    if (c->ev0) cudaEventDestroy(c->ev0);
-    if (c->ev1) cudaEventDestroy(c->ev1);
-    if (c->own_stream) cudaStreamDestroy(c->own_stream);
-    if (c->h_max) cudaFreeHost(c->h_max);
-    delete c;
+    release_context(c);
     return ZK_OK;
 }
 
@@ -231,6 +233,9 @@ int zk_set_mesh(zk_ctx* c, int ny, int nx, double da, double gamma, const int32_
     ZK_CUDA(cudaMalloc(&c->kind, kind.size()));
     ZK_CUDA(cudaMalloc(&c->gsrc, src.size() * sizeof(int32_t)));
     ZK_CUDA(cudaMalloc(&c->d_max, sizeof(MaxSlot)));
+    if (!c->h_max)
+        ZK_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&c->h_max), sizeof *c->h_max,
+                              cudaHostAllocMapped | cudaHostAllocPortable));
     ZK_CUDA(cudaMalloc(&c->d_status, sizeof(uint32_t)));
     ZK_CUDA(cudaMemsetAsync(c->Un, 0, bytes, c->stream));
     ZK_CUDA(cudaMemsetAsync(c->S1, 0, bytes, c->stream));
