@@ -538,8 +538,8 @@ cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s) {
 // Tile by the number of tiles.  Throughput favours 8 rows at 9 warps, 3 CTAs
 // per SM at 72 registers (smaller tiles recompute more halo values per cell,
 // larger ones leave one CTA per SM between its barriers), but a small grid is
-// bound by one tile's latency on a chip mostly idle.  Stage times in us (graph
-// replay; rows/warps x CTAs per SM; tiles of 8 rows):
+// bound by one tile's latency on a chip mostly idle.  Stage times in us on 148
+// SMs (graph replay; rows/warps x CTAs per SM; tiles of 8 rows):
 //            8/9x3  2/14x2  8/18x1  16/26x1
 //   64^2     13.3     6.3     9.7    14.4       16 tiles
 //   128^2    13.4     7.0     9.8    14.5       64
@@ -551,7 +551,6 @@ cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s) {
 // 8, then of 16 rows per SM while that suffices, else 8/9.
 template <int RECON>
 cudaError_t launch_stage(const StageArgs& a, cudaStream_t s) {
-    constexpr int kSms = 148;
     // every tile height at once: a later call with another grid may be inside a
     // stream capture, where no kernel should be loaded for the first time
     static PerContext attributes;
@@ -566,11 +565,15 @@ cudaError_t launch_stage(const StageArgs& a, cudaStream_t s) {
     });
     if (e != cudaSuccess) return e;
     if constexpr (RECON == 0) {
+        int dev = 0, sms = 0;
+        cudaError_t q = cudaGetDevice(&dev);
+        if (q == cudaSuccess) q = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (q != cudaSuccess) return q;
         const long long cols = (a.g.nx + TX - 1) / TX;
         auto tiles = [&](int rows) { return cols * ((a.g.ny + rows - 1) / rows); };
-        if (tiles(2) <= 2 * kSms) return launch_tiles<RECON, 2, 14, 2>(a, s);
-        if (tiles(8) <= kSms) return launch_tiles<RECON, 8, 18, 1>(a, s);
-        if (tiles(16) <= kSms) return launch_tiles<RECON, 16, 26, 1>(a, s);
+        if (tiles(2) <= 2 * sms) return launch_tiles<RECON, 2, 14, 2>(a, s);
+        if (tiles(8) <= sms) return launch_tiles<RECON, 8, 18, 1>(a, s);
+        if (tiles(16) <= sms) return launch_tiles<RECON, 16, 26, 1>(a, s);
     }
     return launch_tiles<RECON, 8, 9, 3>(a, s);
 }

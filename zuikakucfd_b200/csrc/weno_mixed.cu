@@ -506,7 +506,8 @@ cudaError_t launch_tiles(const CUtensorMap& tmap, const MixedArgs& a, cudaStream
 
 // Tile of the single-problem stage on a grid.  Throughput favours 8 rows at 9
 // warps, 5 CTAs per SM; a small grid is bound by the latency of one tile, and
-// its chip by idle SMs.  Stage times in us (graph replay; rows/warps; tiles of 8 rows):
+// its chip by idle SMs.  Stage times in us on 148 SMs (graph replay; rows/warps;
+// tiles of 8 rows):
 //            8/9    8/18   4/10   2/6
 //   64^2      6.4    5.2    5.1    4.7     16 tiles
 //   128^2     7.1    6.3    6.1    5.5     64
@@ -518,18 +519,17 @@ cudaError_t launch_tiles(const CUtensorMap& tmap, const MixedArgs& a, cudaStream
 // so 2 rows while those tiles are all resident at four per SM, 18 warps per
 // 8-row tile up to three tiles per SM, else 9.
 enum class MixedTile { Rows2, Rows8Wide, Rows8 };
-static MixedTile mixed_tile(const Grid& g) {
-    constexpr int kSms = 148;
+static MixedTile mixed_tile(const Grid& g, int sms) {
     const long long cols = (g.nx + TX - 1) / TX;
     auto tiles = [&](int rows) { return cols * ((g.ny + rows - 1) / rows); };
-    if (tiles(2) <= 4 * kSms) return MixedTile::Rows2;
-    return tiles(8) <= 3 * kSms ? MixedTile::Rows8Wide : MixedTile::Rows8;
+    if (tiles(2) <= 4 * sms) return MixedTile::Rows2;
+    return tiles(8) <= 3 * sms ? MixedTile::Rows8Wide : MixedTile::Rows8;
 }
 // Box rows of its tensor maps.
-int weno_mixed_rows(const Grid& g) { return mixed_tile(g) == MixedTile::Rows2 ? 2 : 8; }
+int weno_mixed_rows(const Grid& g, int sms) { return mixed_tile(g, sms) == MixedTile::Rows2 ? 2 : 8; }
 
-static cudaError_t launch_grid(const CUtensorMap& tmap, const MixedArgs& a, cudaStream_t s) {
-    switch (mixed_tile(a.g)) {
+static cudaError_t launch_grid(const CUtensorMap& tmap, const MixedArgs& a, int sms, cudaStream_t s) {
+    switch (mixed_tile(a.g, sms)) {
         case MixedTile::Rows2: return launch_tiles<2, 6, 4>(tmap, a, s);
         case MixedTile::Rows8Wide: return launch_tiles<8, 18, 2>(tmap, a, s);
         default: return launch_tiles<8, 9, 5>(tmap, a, s);
@@ -538,9 +538,10 @@ static cudaError_t launch_grid(const CUtensorMap& tmap, const MixedArgs& a, cuda
 
 cudaError_t launch_weno_stage_mixed(const CUtensorMap& tmap, const double* Ucur, const double* Un, double* Uout,
                                     const int8_t* kind, const int32_t* gsrc, const Grid& g, double dtdx,
-                                    double dtdy, double gamma, int stage, uint32_t* status, cudaStream_t s) {
+                                    double dtdy, double gamma, int stage, uint32_t* status, int sms,
+                                    cudaStream_t s) {
     MixedArgs a{Ucur, Un, Uout, kind, gsrc, g, dtdx, dtdy, gamma, stage, status};
-    return launch_grid(tmap, a, s);
+    return launch_grid(tmap, a, sms, s);
 }
 
 // Stage 1 of the mixed WENO step with a barrier that expects 16 bytes more
@@ -549,9 +550,9 @@ cudaError_t launch_weno_stage_mixed(const CUtensorMap& tmap, const double* Ucur,
 // waits for its copy to land and leaves without writing its tile.
 cudaError_t launch_weno_timeout_selftest(const CUtensorMap& tmap, const double* Un, double* Uout, const int8_t* kind,
                                          const int32_t* gsrc, const Grid& g, double dtdx, double dtdy, double gamma,
-                                         uint32_t spin, uint32_t* status, cudaStream_t s) {
+                                         uint32_t spin, uint32_t* status, int sms, cudaStream_t s) {
     MixedArgs a{Un, Un, Uout, kind, gsrc, g, dtdx, dtdy, gamma, 1, status, 0, 16u, spin ? spin : 1u};
-    return launch_grid(tmap, a, s);
+    return launch_grid(tmap, a, sms, s);
 }
 
 // Tensor map over one FP64 WENO state: dims (x = nx, y = ny, field = 4),
@@ -569,8 +570,9 @@ bool encode_weno_state_map(CUtensorMap* m, const double* base, const Grid& g, co
 int zk_weno_mixed_setup(zk_ctx* c) {
     const char* err = nullptr;
     double* bufs[3] = {c->Un, c->S1, c->S2};
+    const int rows = zk::weno_mixed_rows(c->g, c->sms);
     for (int b = 0; b < 3; ++b)
-        if (!zk::encode_weno_state_map(&c->tmap[b], bufs[b], c->g, &err, zk::weno_mixed_rows(c->g))) return zk_internal_fail(ZK_ERR_CUDA, err);
+        if (!zk::encode_weno_state_map(&c->tmap[b], bufs[b], c->g, &err, rows)) return zk_internal_fail(ZK_ERR_CUDA, err);
     return ZK_OK;
 }
 
@@ -578,13 +580,13 @@ int zk_weno_mixed_step(zk_ctx* c, double dt) {
     const double dtdx = dt / c->da, dtdy = dt / c->da;
     cudaError_t e;
     e = zk::launch_weno_stage_mixed(c->tmap[0], c->Un, c->Un, c->S1, c->kind, c->gsrc, c->g, dtdx, dtdy, c->gamma, 1,
-                                    c->d_status, c->stream);
+                                    c->d_status, c->sms, c->stream);
     if (e == cudaSuccess)
         e = zk::launch_weno_stage_mixed(c->tmap[1], c->S1, c->Un, c->S2, c->kind, c->gsrc, c->g, dtdx, dtdy, c->gamma,
-                                        2, c->d_status, c->stream);
+                                        2, c->d_status, c->sms, c->stream);
     if (e == cudaSuccess)
         e = zk::launch_weno_stage_mixed(c->tmap[2], c->S2, c->Un, c->Un, c->kind, c->gsrc, c->g, dtdx, dtdy, c->gamma,
-                                        3, c->d_status, c->stream);
+                                        3, c->d_status, c->sms, c->stream);
     if (e != cudaSuccess) return zk_internal_fail(ZK_ERR_CUDA, cudaGetErrorString(e));
     return ZK_OK;
 }
@@ -597,7 +599,7 @@ extern "C" int zk_selftest_tma_timeout(zk_ctx* c, uint32_t spin_limit, uint32_t*
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, sizeof(uint32_t), c->stream);
     if (e == cudaSuccess)
         e = zk::launch_weno_timeout_selftest(c->tmap[0], c->Un, c->S1, c->kind, c->gsrc, c->g, 1e-6 / c->da,
-                                             1e-6 / c->da, c->gamma, spin_limit, c->d_status, c->stream);
+                                             1e-6 / c->da, c->gamma, spin_limit, c->d_status, c->sms, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(status_out, c->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -612,6 +614,6 @@ int zk_weno_mixed_stage(zk_ctx* c, double dt, int stage) {
     double* out[3] = {c->S1, c->S2, c->Un};
     const cudaError_t e = zk::launch_weno_stage_mixed(c->tmap[stage - 1], in[stage - 1], c->Un, out[stage - 1], c->kind,
                                                       c->gsrc, c->g, dtdx, dtdy, c->gamma, stage, c->d_status,
-                                                      c->stream);
+                                                      c->sms, c->stream);
     return e == cudaSuccess ? ZK_OK : zk_internal_fail(ZK_ERR_CUDA, cudaGetErrorString(e));
 }
