@@ -2,12 +2,20 @@
 //
 // The runtime stages a pageable copy through one page-locked buffer on one
 // host thread: to a fresh host array (numpy's, whose pages fault on the way)
-// 4.5 GB/s, from one 11 to 16.  Large copies are dealt to kWorkers host
-// threads instead, each moving its share through two page-locked buffers of
-// its own, so that one fills or empties while the other is in flight.  Reading
-// a 75 MB state 17.3 -> 4.7 ms, 537 MB 116 -> 25; setting them 6.5 -> 3.3 and 49
-// -> 19.  The first staged copy of a context page-locks 5 MB (3 to 5 ms), so
-// uploads, which lose less to the runtime, do not start it below 192 MB.
+// 2 GB/s.  Large copies are dealt to kWorkers host threads instead, each moving
+// its share through two page-locked buffers of its own, so that one fills or
+// empties while the other is in flight.  Milliseconds, plain and staged; "warm"
+// is an array whose pages are there, and odd row lengths slow the plain copy:
+//            read, fresh     read, warm     upload
+//    32 MB   17.4 / 5.9      3.5 / 1.7      3.6 / 2.8
+//    48 MB   23.0 / 8.7      2.4 / 2.5      3.7 / 3.4
+//    96 MB   50   / 17       8.0 / 4.7     12   / 5.9
+//   192 MB   92   / 34       9.0 / 9.0     17   / 8.9
+//   400 MB  202   / 72      18.9 / 19      40   / 20
+// The buffers are 1.5 MB in all: page-locking those costs next to nothing, 2 MB
+// 2 ms and 5 MB (five workers, 512 KB each) 4 to 5 ms at the first copy, more
+// than a warm copy below 100 MB gains.  Their release adds 0.6 ms to the
+// context's.
 //
 // The workers' copies run on a stream of the staging's own, behind an event of
 // the caller's: a stream handle may mean another stream in another thread
@@ -26,10 +34,9 @@
 namespace zk {
 namespace {
 
-constexpr int kWorkers = 5;
-constexpr size_t kChunk = size_t(512) << 10;      // bytes of one staging buffer
-constexpr size_t kStagedMin = size_t(4) << 20;    // smaller copies are not worth the threads
-constexpr size_t kAllocMin = size_t(24) << 20;    // nor smaller ones page-locking the buffers
+constexpr int kWorkers = 3;
+constexpr size_t kChunk = size_t(256) << 10;    // bytes of one staging buffer
+constexpr size_t kStagedMin = size_t(32) << 20;  // smaller copies lose to the plain one where it is fast
 
 // Exempts this thread from the calls that another stream's capture forbids
 // (page-locking memory, waiting for an event): none of them concerns it.
@@ -108,9 +115,8 @@ bool HostStage::allocate() {
     return false;
 }
 
-bool HostStage::ready(bool to_device, const void* host, size_t bytes, size_t width, cudaStream_t s) {
-    if (width > kChunk || bytes < (base_ ? kStagedMin : kAllocMin) || (to_device && !base_ && bytes < 8 * kAllocMin))
-        return false;
+bool HostStage::ready(const void* host, size_t bytes, size_t width, cudaStream_t s) {
+    if (width > kChunk || bytes < kStagedMin) return false;
     cudaPointerAttributes at;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaPointerGetAttributes(&at, host) != cudaSuccess || cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
@@ -123,7 +129,7 @@ bool HostStage::ready(bool to_device, const void* host, size_t bytes, size_t wid
 
 template <bool TO_DEVICE>
 cudaError_t HostStage::copy(char* host, char* dev, size_t pitch, size_t width, size_t rows, cudaStream_t s) {
-    if (!ready(TO_DEVICE, host, width * rows, width, s)) {
+    if (!ready(host, width * rows, width, s)) {
         const cudaError_t e =
             TO_DEVICE ? cudaMemcpy2DAsync(dev, pitch, host, width, width, rows, cudaMemcpyHostToDevice, s)
                       : cudaMemcpy2DAsync(host, width, dev, pitch, width, rows, cudaMemcpyDeviceToHost, s);

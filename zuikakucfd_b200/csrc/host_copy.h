@@ -25,7 +25,7 @@ public:
 private:
     template <bool TO_DEVICE>
     cudaError_t copy(char* host, char* dev, size_t pitch, size_t width, size_t rows, cudaStream_t s);
-    bool ready(bool to_device, const void* host, size_t bytes, size_t width, cudaStream_t s);
+    bool ready(const void* host, size_t bytes, size_t width, cudaStream_t s);
     bool allocate();
     char* base_ = nullptr;
     cudaStream_t stream_ = nullptr;
