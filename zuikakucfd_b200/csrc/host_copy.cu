@@ -12,10 +12,10 @@
 //    96 MB   50   / 17       8.0 / 4.7     12   / 5.9
 //   192 MB   92   / 34       9.0 / 9.0     17   / 8.9
 //   400 MB  202   / 72      18.9 / 19      40   / 20
-// The buffers are 1.5 MB in all: page-locking those costs next to nothing, 2 MB
-// 2 ms and 5 MB (five workers, 512 KB each) 4 to 5 ms at the first copy, more
-// than a warm copy below 100 MB gains.  Their release adds 0.6 ms to the
-// context's.
+// The buffers are 1.5 MB in all: page-locking them takes 1 to 3 ms (nothing where
+// other page-locked memory is about; 5 MB, five workers with 512 KB each, 4 to
+// 5 ms), which the first staged copy pays, so that one starts at kFirstMin.
+// Their release adds 0.6 ms to the context's.
 //
 // The workers' copies run on a stream of the staging's own, behind an event of
 // the caller's: a stream handle may mean another stream in another thread
@@ -37,6 +37,7 @@ namespace {
 constexpr int kWorkers = 3;
 constexpr size_t kChunk = size_t(256) << 10;    // bytes of one staging buffer
 constexpr size_t kStagedMin = size_t(32) << 20;  // smaller copies lose to the plain one where it is fast
+constexpr size_t kFirstMin = size_t(64) << 20;   // as does one that makes the buffers
 
 // Exempts this thread from the calls that another stream's capture forbids
 // (page-locking memory, waiting for an event): none of them concerns it.
@@ -116,7 +117,7 @@ bool HostStage::allocate() {
 }
 
 bool HostStage::ready(const void* host, size_t bytes, size_t width, cudaStream_t s) {
-    if (width > kChunk || bytes < kStagedMin) return false;
+    if (width > kChunk || bytes < (base_ ? kStagedMin : kFirstMin)) return false;
     cudaPointerAttributes at;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaPointerGetAttributes(&at, host) != cudaSuccess || cudaStreamIsCapturing(s, &cs) != cudaSuccess) {

@@ -8,6 +8,8 @@
 #include <cstring>
 #include <fstream>
 #include <string>
+#include <sys/mman.h>
+#include <unistd.h>
 #include <vector>
 
 #include "zk_common.cuh"
@@ -54,12 +56,39 @@ void free_device(zk_ctx* c) {
     c->d_status = nullptr;
 }
 
+// One page of host memory, page-locked and visible to the device at the same
+// address, left out of forked processes (a fork could move it from under the
+// device).  cudaHostAlloc takes 2 MB from the system for 8 bytes: a context's
+// first mesh 1.4 to 2.4 ms longer and its end 0.4, with this page 0.3 and 0.2.
+cudaError_t page_locked_alloc(void** p) {
+    const size_t page = sysconf(_SC_PAGESIZE);
+    void* m = mmap(nullptr, page, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (m == MAP_FAILED) return cudaErrorMemoryAllocation;
+    madvise(m, page, MADV_DONTFORK);
+    cudaError_t e = cudaHostRegister(m, page, cudaHostRegisterMapped | cudaHostRegisterPortable);
+    if (e == cudaSuccess) {
+        void* d = nullptr;
+        e = cudaHostGetDevicePointer(&d, m, 0);
+        if (e == cudaSuccess && d != m) e = cudaErrorNotSupported;
+        if (e != cudaSuccess) cudaHostUnregister(m);
+    }
+    if (e != cudaSuccess) munmap(m, page);
+    else *p = m;
+    return e;
+}
+
+void page_locked_free(void* p) {
+    if (!p) return;
+    cudaHostUnregister(p);
+    munmap(p, sysconf(_SC_PAGESIZE));
+}
+
 // What zk_create made (and h_max, made with the first mesh), and the context.
 void release_context(zk_ctx* c) {
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
-    if (c->h_max) cudaFreeHost(c->h_max);
+    page_locked_free(c->h_max);
     delete c;
 }
 
@@ -233,9 +262,7 @@ int zk_set_mesh(zk_ctx* c, int ny, int nx, double da, double gamma, const int32_
     ZK_CUDA(cudaMalloc(&c->kind, kind.size()));
     ZK_CUDA(cudaMalloc(&c->gsrc, src.size() * sizeof(int32_t)));
     ZK_CUDA(cudaMalloc(&c->d_max, sizeof(MaxSlot)));
-    if (!c->h_max)
-        ZK_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&c->h_max), sizeof *c->h_max,
-                              cudaHostAllocMapped | cudaHostAllocPortable));
+    if (!c->h_max) ZK_CUDA(page_locked_alloc(reinterpret_cast<void**>(&c->h_max)));
     ZK_CUDA(cudaMalloc(&c->d_status, sizeof(uint32_t)));
     ZK_CUDA(cudaMemsetAsync(c->Un, 0, bytes, c->stream));
     ZK_CUDA(cudaMemsetAsync(c->S1, 0, bytes, c->stream));
