@@ -509,21 +509,21 @@ cudaError_t launch_tiles(const CUtensorMap& tmap, const MixedArgs& a, cudaStream
 // its chip by idle SMs.  Stage times in us on 148 SMs (graph replay; rows/warps;
 // tiles of 8 rows):
 //            8/9    8/18   4/10   2/6
-//   64^2      6.4    5.2    5.1    4.7     16 tiles
-//   128^2     7.1    6.3    6.1    5.5     64
-//   192^2     8.8    6.0    6.6    5.8    144
-//   256^2    11.3    6.9    8.9    9.2    256
-//   300^2    12.3    9.6   10.5   12.1    380
-//   400^2    12.8   14.0   15.6   18.4    650
-//   1024^2   55.3   72.7   86.1  108     4096
-// so 2 rows while those tiles are all resident at four per SM, 18 warps per
-// 8-row tile up to three tiles per SM, else 9.
+//   64^2      6.1    4.9    4.8    4.4     16 tiles
+//   128^2     6.2    5.0    5.0    4.9     64
+//   192^2     6.2    5.0    5.4    5.7    144
+//   256^2     7.8    6.7    8.7    9.2    256
+//   300^2     9.2    9.4   10.4   12.2    380
+//   400^2    12.4   13.7   15.5   18.6    650
+//   1024^2   55.6   72.6   86.1  108     4096
+// so 2 rows up to two such tiles per SM, 18 warps per 8-row tile up to two of
+// those per SM, else 9.
 enum class MixedTile { Rows2, Rows8Wide, Rows8 };
 static MixedTile mixed_tile(const Grid& g, int sms) {
     const long long cols = (g.nx + TX - 1) / TX;
     auto tiles = [&](int rows) { return cols * ((g.ny + rows - 1) / rows); };
-    if (tiles(2) <= 4 * sms) return MixedTile::Rows2;
-    return tiles(8) <= 3 * sms ? MixedTile::Rows8Wide : MixedTile::Rows8;
+    if (tiles(2) <= 2 * sms) return MixedTile::Rows2;
+    return tiles(8) <= 2 * sms ? MixedTile::Rows8Wide : MixedTile::Rows8;
 }
 // Box rows of its tensor maps.
 int weno_mixed_rows(const Grid& g, int sms) { return mixed_tile(g, sms) == MixedTile::Rows2 ? 2 : 8; }
