@@ -231,7 +231,7 @@ __device__ __noinline__ void hllc_dg_any(const double* L, const double* R, doubl
 // The same flux, quotients over a common denominator sharing its reciprocal:
 // the same values formed in the same order.  Its 15 divisions and 6 square
 // roots are over half of an interface's FP64 work (face pass with plain
-// division: P=3 1024^2 419 us, now 370; contracted build 768^2 269, now 196).
+// division: P=3 1024^2 419 us, now 373; contracted build 768^2 269, now 207).
 __device__ __forceinline__ void hllc_dg(const double (&L)[4], const double (&R)[4], double gamma, double (&F)[4]) {
     const double eps = 1e-5;
     const double rhoL = ref_max(L[0], eps), rhoR = ref_max(R[0], eps);
@@ -458,8 +458,8 @@ __global__ void __launch_bounds__(FaceTile<P>::NTHREAD) dg_face_kernel(DGArgs a,
 // whole 256-byte row segments, its table reads are warp-uniform.  With one
 // thread per cell the 64 accumulators of P = 3 spilled 656 bytes and the face
 // fluxes arrived in 16 dependent rounds of loads (P=3 1024^2: 2,093 us, FP64
-// pipe 28%); now 720 us (FP64 pipe 66%).  The same layout at P=2 203x331: 69 ->
-// 32 us.
+// pipe 28%); now 722 us (FP64 pipe 68%).  The same layout at P=2 203x331: 69 ->
+// 30 us.
 template <int P>
 struct CellTile {
     static constexpr int NQ = P + 1, NM = NQ * NQ, NTHREAD = 32 * NQ;
@@ -745,7 +745,7 @@ __device__ __forceinline__ void integrals(const DGTab& T, CellTile<P>& S, double
 // take 768.  With one fused launch per stage (two threads per cell, tile and
 // interface fluxes in one CTA: 208 registers, 8 warps per SM, FP64 pipe 23%)
 // the P=3 stage at 768^2 took 1,077 us, this pass and the face pass take
-// 517.
+// 535.
 template <int P>
 __device__ __forceinline__ void integrals_factored(const DGTab& T, CellTile<P>& S, double gamma,
                                                    double (&o)[4][P + 1]) {

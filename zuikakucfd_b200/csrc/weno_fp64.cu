@@ -20,8 +20,8 @@
 // (the same expressions of the same cells), so the reconstruction runs per
 // cell: 3 indicators, 3 reciprocals and 5 weights where a face evaluates 6, 6
 // and 6; and every division is branch-free (fp64_div.cuh).  About 1,070 FP64
-// instructions per interface become 780: 177 -> 156 us a stage at 1024^2 (FP64
-// pipe 64%; the staging, combine and barrier phases of three CTAs per SM leave
+// instructions per interface become 805: 177 -> 159 us a stage at 1024^2 (FP64
+// pipe 65%; the staging, combine and barrier phases of three CTAs per SM leave
 // the rest).
 #include "batch.cuh"
 #include "chain.cuh"
@@ -541,12 +541,12 @@ cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s) {
 // bound by one tile's latency on a chip mostly idle.  Stage times in us on 148
 // SMs (graph replay; rows/warps x CTAs per SM; tiles of 8 rows):
 //            8/9x3  2/14x2  8/18x1  16/26x1
-//   64^2     13.3     6.3     9.7    14.4       16 tiles
-//   128^2    13.4     7.0     9.8    14.5       64
-//   192^2    13.4    13.0     9.8    14.6      144
-//   256^2    16.7    21.0    17.3    14.6      256
-//   300^2    21.3    28.2    24.5    26.8      380
-//   1024^2  154     313     223     184       4096
+//   64^2     11.8     5.4     9.8    14.2       16 tiles
+//   128^2    12.0     7.3    10.1    14.6       64
+//   192^2    12.3    13.1    10.1    14.6      144
+//   256^2    16.8    21.7    18.0    14.6      256
+//   300^2    21.4    29.7    25.7    27.1      380
+//   1024^2  158     331     246     188       4096
 // so the 2-row tile while two per SM are all resident, then one wider tile of
 // 8, then of 16 rows per SM while that suffices, else 8/9.
 template <int RECON>
