@@ -47,7 +47,7 @@ struct zk_ctx {
     int dg_tpc = 0;               // threads per cell of the mixed DG stage kernel (0: not chosen yet)
     int32_t* d_list = nullptr;    // cells the fused indicator flagged in the current stage (pitched indices)
     uint32_t* d_lcount = nullptr; // their counts, one per RK stage, cleared at each step's stage 1
-    uint8_t* d_flags = nullptr;   // TVB troubled-cell flags of the last pass, pitched
+    uint8_t* d_flags = nullptr;   // troubled-cell flags of the feature-extraction passes, pitched
     uint32_t* d_nflag = nullptr;  // cells the TVB passes limited during the last zk_step
 
     cudaGraphExec_t step_graph = nullptr;  // kGraphSteps steps at step_graph_dt (zk_step)
