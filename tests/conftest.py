@@ -16,6 +16,12 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200) and the built native library")
 
 
+def pytest_collection_modifyitems(items):
+    """The drop-in tests fail where the reference's own binaries are not built:
+    last, so that with -x every other test has run."""
+    items.sort(key=lambda item: item.path.name == "test_dropin_gpu.py")
+
+
 @pytest.fixture(scope="session")
 def golden():
     z = np.load(GOLDEN / "reference_golden.npz")
