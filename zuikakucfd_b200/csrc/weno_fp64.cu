@@ -548,7 +548,10 @@ cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s) {
 //   300^2    21.4    29.7    25.7    27.1      380
 //   1024^2  158     331     246     188       4096
 // so the 2-row tile while two per SM are all resident, then one wider tile of
-// 8, then of 16 rows per SM while that suffices, else 8/9.
+// 8, then of 16 rows per SM while that suffices, else 8/9.  Tile rows of ghosts
+// alone do not count (33 x 1024: 9.8 us with 8/18, 13.4 with 16/26), and a grid
+// just above one 8-row tile per SM stays with 8/9 while its updated rows would
+// fit one (39 x 960: 12.1 against 14.5; 163 x 250, which does not: 16.2, 14.6).
 template <int RECON>
 cudaError_t launch_stage(const StageArgs& a, cudaStream_t s) {
     // every tile height at once: a later call with another grid may be inside a
@@ -570,10 +573,10 @@ cudaError_t launch_stage(const StageArgs& a, cudaStream_t s) {
         if (q == cudaSuccess) q = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (q != cudaSuccess) return q;
         const long long cols = (a.g.nx + TX - 1) / TX;
-        auto tiles = [&](int rows) { return cols * ((a.g.ny + rows - 1) / rows); };
+        auto tiles = [&](int rows) { return cols * ((a.g.ny - 3 + rows - 1) / rows); };
         if (tiles(2) <= 2 * sms) return launch_tiles<RECON, 2, 14, 2>(a, s);
         if (tiles(8) <= sms) return launch_tiles<RECON, 8, 18, 1>(a, s);
-        if (tiles(16) <= sms) return launch_tiles<RECON, 16, 26, 1>(a, s);
+        if (cols * (a.g.ny - 6) > 8 * sms && tiles(16) <= sms) return launch_tiles<RECON, 16, 26, 1>(a, s);
     }
     return launch_tiles<RECON, 8, 9, 3>(a, s);
 }
