@@ -352,19 +352,25 @@ __device__ __forceinline__ void copy_wait() {
 // and serve both directions (a thread per face and direction read each cell
 // twice from L2, and its 4 NQ traces took 128-146 registers: 4 CTAs of 4 warps
 // per SM, FP64 pipe 40-45%).
-template <int P>
+
+// Gauss points per thread (a throughput choice: P = 3, 1024^2: 2 373 us, 1 475,
+// 4 495).  A grid of few CTAs is bound by the latency of a thread's interface
+// fluxes instead and takes one point per thread, see launch_stage.
+constexpr int face_points(int P) { return P == 3 ? 2 : P + 1; }
+
+template <int P, int QPT = face_points(P)>
 struct FaceTile {
     static constexpr int NQ = P + 1, NM = NQ * NQ;
-    static constexpr int QP = P == 3 ? 2 : NQ;  // Gauss points per thread
-    static constexpr int NWD = NQ / QP;         // warps per direction
+    static constexpr int QP = QPT;       // Gauss points per thread
+    static constexpr int NWD = NQ / QP;  // warps per direction
     static constexpr int NTHREAD = 64 * NWD;
     double lo[4 * NM][34];  // row i, columns j0-1 .. j0+31
     double up[4 * NM][32];  // row i-1, columns j0 .. j0+31
 };
 
-template <int P>
-__device__ __forceinline__ void face_tile(const DGArgs& a, int j0, int i, FaceTile<P>& S) {
-    using F = FaceTile<P>;
+template <int P, int QPT>
+__device__ __forceinline__ void face_tile(const DGArgs& a, int j0, int i, FaceTile<P, QPT>& S) {
+    using F = FaceTile<P, QPT>;
     constexpr int NM = F::NM, QP = F::QP, NW = F::NTHREAD / 32;
     const DGTab& T = c_dgtab[P - 1];
     const int ny = a.g.ny, nx = a.g.nx, pitch = a.g.pitch;
@@ -441,11 +447,11 @@ __device__ __forceinline__ void face_tile(const DGArgs& a, int j0, int i, FaceTi
 
 // Rows 3 .. ny-3 hold every face of an updated cell; TALL: from row `row0`, a
 // variant of its own since the addition alone made the pass 1 to 4% longer.
-template <int P, bool TALL>
-__global__ void __launch_bounds__(FaceTile<P>::NTHREAD) dg_face_kernel(DGArgs a, int row0) {
-    __shared__ FaceTile<P> S;
+template <int P, bool TALL, int QPT = face_points(P)>
+__global__ void __launch_bounds__(FaceTile<P, QPT>::NTHREAD) dg_face_kernel(DGArgs a, int row0) {
+    __shared__ FaceTile<P, QPT> S;
     chain_wait();
-    face_tile<P>(a, blockIdx.x * 32, (TALL ? row0 : 3) + blockIdx.y, S);
+    face_tile(a, blockIdx.x * 32, (TALL ? row0 : 3) + blockIdx.y, S);
 }
 
 // ---- cells ---------------------------------------------------------------------------
@@ -1030,7 +1036,7 @@ __global__ void __launch_bounds__(FaceTile<P>::NTHREAD, P == 3 ? 5 : 8) dg_faces
             }
         }
         __syncthreads();
-        if (s_job[0]) face_tile<P>(sa, s_job[2], s_job[1], S);
+        if (s_job[0]) face_tile(sa, s_job[2], s_job[1], S);
         __syncthreads();
     }
 }
@@ -1090,13 +1096,27 @@ __global__ void __launch_bounds__(CellTile<P>::NTHREAD) dg_limit_kernel(DGArgs a
             for (int n = 0; n < NQ; ++n) a.out[(size_t)(c * NM + CellTile<P>::mode(w, n)) * plane + k] = o[c][n];
 }
 
+// One Gauss point per thread while the face pass has at most two CTAs per SM
+// (a step on 148 SMs, us, several points and one; FP64 and FP64_FMA):
+//             CTAs   P=1                    P=2                    P=3
+//   64^2       118   31.3 27.4  28.5 25.1   43.9 36.0  38.2 31.1   51.7 47.9  40.2 37.3
+//   96^2       273   31.1 27.7  28.7 25.6   46.1 39.2  39.8 33.8   56.7 55.9  45.7 45.1
+//   128^2      492   32.5 31.1  30.7 29.6   50.4 49.4  45.6 48.6   85.1 86.6  65.9 71.4
+//   192^2     1122   42.0 43.4  41.0 43.2   84.0 86.2  73.0 81.2   151  157   117  134
 template <int P>
 cudaError_t launch_stage(const DGArgs& a, cudaStream_t s) {
     constexpr int kRows = 65535;  // gridDim.y
     const int segs = (a.g.nx + 31) / 32, ny = a.g.ny, faces = ny - 5;
-    cudaError_t e = cudaSuccess;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
     if (ny <= kRows) {
-        e = launch_chained(dg_face_kernel<P, false>, dim3(segs, faces), FaceTile<P>::NTHREAD, 0, s, a, 0);
+        const dim3 grid(segs, faces);
+        if ((long long)segs * faces <= 2 * sms)
+            e = launch_chained(dg_face_kernel<P, false, 1>, grid, FaceTile<P, 1>::NTHREAD, 0, s, a, 0);
+        else
+            e = launch_chained(dg_face_kernel<P, false>, grid, FaceTile<P>::NTHREAD, 0, s, a, 0);
         if (e != cudaSuccess) return e;
         return launch_chained(dg_cell_kernel<P, false>, dim3(segs, ny), CellTile<P>::NTHREAD, 0, s, a, 0);
     }
