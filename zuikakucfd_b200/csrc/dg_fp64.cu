@@ -464,8 +464,8 @@ __global__ void __launch_bounds__(FaceTile<P, QPT>::NTHREAD) dg_face_kernel(DGAr
 // whole 256-byte row segments, its table reads are warp-uniform.  With one
 // thread per cell the 64 accumulators of P = 3 spilled 656 bytes and the face
 // fluxes arrived in 16 dependent rounds of loads (P=3 1024^2: 2,093 us, FP64
-// pipe 28%); now 722 us (FP64 pipe 68%).  The same layout at P=2 203x331: 69 ->
-// 30 us.
+// pipe 28%); now 727 us (FP64 pipe 68%).  The same layout at P=2 203x331: 69 ->
+// 29 us.
 template <int P>
 struct CellTile {
     static constexpr int NQ = P + 1, NM = NQ * NQ, NTHREAD = 32 * NQ;
@@ -473,6 +473,7 @@ struct CellTile {
     double sd[4 * NM][32];      // filled stage input; later the limiter's view of the result
     double fg[CH * NQ][8][32];  // F and G at the round's points; later the limiter's exchange
     double fx[4 * NQ][33], fyu[4 * NQ][32], fyd[4 * NQ][32];  // interface fluxes
+    int bad[NQ][32];  // by eta index: variables with an F (bit c) or G (bit 4 + c) that is not finite
     // mode of thread (lane, w)'s n-th accumulator: px = w in the reference's
     // summation order, py = w where the sums are factorised
     static __device__ __forceinline__ int mode(int w, int n) { return kFma ? n * NQ + w : w * NQ + n; }
@@ -636,6 +637,7 @@ template <int P>
 __device__ __forceinline__ void integrals(const DGTab& T, CellTile<P>& S, double gamma, double (&o)[4][P + 1]) {
     constexpr int NQ = P + 1, NM = NQ * NQ, CH = CellTile<P>::CH;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int bad = 0;
     // volume integral (src_DG/fluid.cpp:698-718), CH rows of points at a time
 #pragma unroll 1
     for (int qa0 = 0; qa0 < NQ; qa0 += CH) {
@@ -656,16 +658,21 @@ __device__ __forceinline__ void integrals(const DGTab& T, CellTile<P>& S, double
         for (int u = 0; u < CH; ++u) {
             double F[4], G[4];
             euler_flux(U[u], gamma, F, G);
+            int top = 0;  // the largest exponent
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 S.fg[u * NQ + w][c][lane] = F[c];
                 S.fg[u * NQ + w][4 + c][lane] = G[c];
+                top = max(top, max(__double2hiint(F[c]) & 0x7fffffff, __double2hiint(G[c]) & 0x7fffffff));
             }
+            if (top >= 0x7ff00000)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) bad |= (isfinite(F[c]) ? 0 : 1 << c) | (isfinite(G[c]) ? 0 : 16 << c);
         }
         __syncthreads();
         // terms whose basis derivative is 0 identically (d/dxi at px = 0,
-        // d/deta at py = 0) add +-0 and are left out, but for mode 0, whose
-        // sum still turns NaN on a non-finite flux as the reference's does
+        // d/deta at py = 0) add +-0 and are left out, or NaN for a flux that is
+        // not finite: those are added at the end, from `bad`
 #pragma unroll 1
         for (int pt = 0; pt < CH * NQ; ++pt) {
             const int p = qa0 * NQ + pt;
@@ -677,8 +684,6 @@ __device__ __forceinline__ void integrals(const DGTab& T, CellTile<P>& S, double
                 G[c] = S.fg[pt][4 + c][lane];
             }
             if (w == 0) {
-#pragma unroll
-                for (int c = 0; c < 4; ++c) o[c][0] += coeff * (F[c] * 0.0 + G[c] * 0.0);
 #pragma unroll
                 for (int n = 1; n < NQ; ++n) {
                     const double det = T.vdet[p][n];
@@ -699,8 +704,17 @@ __device__ __forceinline__ void integrals(const DGTab& T, CellTile<P>& S, double
         }
         if (qa0 + CH < NQ) __syncthreads();
     }
+    S.bad[w][lane] = bad;
     copy_wait<0>();
     __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) bad |= S.bad[q][lane];
+    if (bad)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int n = 0; n < NQ; ++n)
+                if ((w == 0 && (bad >> c & 1)) || (n == 0 && (bad >> (4 + c) & 1))) o[c][n] = NAN;
     // face integrals: right (-), left (+), bottom (-), top (+)
     // (src_DG/fluid.cpp:731-796).  P_n(+1) = 1 and P_n(-1) = (-1)^n exactly,
     // so an x face's weights are those of px = 0 up to sign, and a y face's
